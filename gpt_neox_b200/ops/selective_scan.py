@@ -3,9 +3,10 @@
     delta = softplus(dt + dt_bias);  h_t = exp(delta_t A) * h_{t-1} + delta_t B_t u_t;  y_t = C_t . h_t + D u_t
     out = y * silu(z)
 
-Layouts are channel-last -- u, dt, z ``[b, l, d]``, B, C ``[b, l, n]`` -- so consecutive threads of the CUDA
-kernel (``csrc/selective_scan.cu``, one thread per channel, state in registers, checkpointed every 32 steps for
-the backward recomputation) touch consecutive addresses and no ``b d l`` transposes are needed.
+Layouts are channel-last -- u, dt, z ``[b, l, d]``, B, C ``[b, l, n]``, with any batch and time strides -- so consecutive
+threads of the CUDA kernels (``csrc/selective_scan.cu``: chunks of 32 steps side by side, combined in a short pass; their
+start states are the checkpoints of the backward recomputation) touch consecutive addresses and no ``b d l`` transposes
+are needed.
 ``selective_scan_ref`` states the same recurrence in PyTorch (CPU path and oracle).
 Reference: mamba_ssm ``selective_scan_fn`` / ``causal_conv1d_fn`` as called from ``megatron/model/mamba/mamba.py:207-300``.
 """
@@ -43,20 +44,32 @@ def selective_scan_ref(u, dt, A, B, C, D=None, z=None, dt_bias=None, dt_softplus
     return y.to(u.dtype)
 
 
+def _rows(t, dtype=None):
+    """``t`` ([b, l, x], any batch and time strides) with a contiguous last dimension, as the kernels read it."""
+    t = t if dtype is None else t.to(dtype)
+    return t if t.stride(2) == 1 else t.contiguous()
+
+
+def _strides(*ts):
+    return (ctypes.c_longlong * (2 * len(ts)))(*[s for t in ts for s in t.stride()[:2]])
+
+
 class _Scan(torch.autograd.Function):
     @staticmethod
     def forward(ctx, u, dt, A, B, C, D, z, dt_bias):
         b, l, d = u.shape
         n = A.shape[1]
-        u, dt, z = u.contiguous(), dt.contiguous(), z.contiguous()
-        Bc, Cc = B.float().contiguous(), C.float().contiguous()
+        u, dt, z = _rows(u), _rows(dt), _rows(z)
+        Bc, Cc = _rows(B, torch.float32), _rows(C, torch.float32)
         Af, Df, bias = A.float().contiguous(), D.float().contiguous(), dt_bias.float().contiguous()
         nchk = (l + 31) // 32
         y = torch.empty_like(u)
-        ckpt = torch.empty(b, nchk, d, n, dtype=torch.float32, device=u.device)
+        ckpt = torch.empty(b, nchk, n, d, dtype=torch.float32, device=u.device)
+        sumd = torch.empty(b, nchk, d, dtype=torch.float32, device=u.device)
         rc = native.lib().neox_selective_scan_fwd(native.ptr(u), native.ptr(dt), native.ptr(Af), native.ptr(Bc),
                                                   native.ptr(Cc), native.ptr(Df), native.ptr(z), native.ptr(bias),
-                                                  native.ptr(y), native.ptr(ckpt), b, l, d, n,
+                                                  native.ptr(y), native.ptr(ckpt), native.ptr(sumd),
+                                                  _strides(u, dt, z, y, Bc, Cc), b, l, d, n,
                                                   ctypes.c_void_p(native.stream_ptr()))
         native.check(rc, "neox_selective_scan_fwd")
         ctx.save_for_backward(u, dt, Af, Bc, Cc, Df, z, bias, ckpt)
@@ -68,18 +81,18 @@ class _Scan(torch.autograd.Function):
         u, dt, Af, Bc, Cc, Df, z, bias, ckpt = ctx.saved_tensors
         b, l, d = u.shape
         n = Af.shape[1]
-        gy = gy.contiguous()
+        gy = _rows(gy)
         du, ddt, dz = torch.empty_like(u), torch.empty_like(dt), torch.empty_like(z)
-        dA = torch.zeros(d, n, dtype=torch.float32, device=u.device)
-        dB = torch.zeros(b, l, n, dtype=torch.float32, device=u.device)
-        dC = torch.zeros(b, l, n, dtype=torch.float32, device=u.device)
-        dD = torch.zeros(d, dtype=torch.float32, device=u.device)
-        dbias = torch.zeros(d, dtype=torch.float32, device=u.device)
+        sums = torch.zeros(d * n + 2 * b * l * n + 2 * d, dtype=torch.float32, device=u.device)
+        dA, dB, dC, dD, dbias = sums.split([d * n, b * l * n, b * l * n, d, d])
+        dA, dB, dC = dA.view(d, n), dB.view(b, l, n), dC.view(b, l, n)
+        gst, sumd = torch.empty_like(ckpt), torch.empty(b, ckpt.shape[1], d, dtype=torch.float32, device=u.device)
         rc = native.lib().neox_selective_scan_bwd(native.ptr(u), native.ptr(dt), native.ptr(Af), native.ptr(Bc),
                                                   native.ptr(Cc), native.ptr(Df), native.ptr(z), native.ptr(bias),
                                                   native.ptr(ckpt), native.ptr(gy), native.ptr(du), native.ptr(ddt),
                                                   native.ptr(dz), native.ptr(dA), native.ptr(dB), native.ptr(dC),
-                                                  native.ptr(dD), native.ptr(dbias), b, l, d, n,
+                                                  native.ptr(dD), native.ptr(dbias), native.ptr(gst), native.ptr(sumd),
+                                                  _strides(u, dt, z, gy, Bc, Cc, du, ddt, dz, dB), b, l, d, n,
                                                   ctypes.c_void_p(native.stream_ptr()))
         native.check(rc, "neox_selective_scan_bwd")
         ta, tb, tc, td, tbias = ctx.dtypes

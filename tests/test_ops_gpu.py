@@ -989,3 +989,33 @@ def test_squared_norm_kernel_any_alignment(n, offset):
     native.check(rc, "neox_sumsq_f32")
     ref = (x.double() ** 2).sum().item()
     assert abs(out.item() - ref) <= 2e-5 * max(ref, 1.0), (out.item(), ref)
+
+
+@pytest.mark.parametrize("b,l,d,time_major", [(1, 1, 64, False), (2, 33, 65, True), (3, 96, 136, True), (1, 300, 40, False),
+                                              (2, 40, 75776, False)])
+def test_selective_scan_chunks_and_strides(b, l, d, time_major):
+    """Edges of the chunked scan -- one step, a chunk and one step, whole chunks, many chunks, channels that leave a block
+    part full, channels that fill the machine (no split of time) -- on operands that are slices of wider [l, b, ...]
+    tensors, against the recurrence in fp32.  bf16 outputs: half an ulp (2^-9) of the value plus the summation error."""
+    from gpt_neox_b200.ops import selective_scan as SS
+    torch.manual_seed(l)
+    n = 16
+
+    def mk(w, dtype, scale=1.0):
+        t = (torch.randn(l, b, w + 8, device=DEV) * scale).to(dtype)[..., 8:].transpose(0, 1) if time_major \
+            else (torch.randn(b, l, w, device=DEV) * scale).to(dtype)
+        return t.detach().requires_grad_(True)
+    u, dt, z = mk(d, torch.bfloat16), mk(d, torch.bfloat16, 0.5), mk(d, torch.bfloat16)
+    B, C = mk(n, torch.float32, 0.5), mk(n, torch.float32, 0.5)
+    A = (-torch.rand(d, n, device=DEV) * 2 - 0.1).requires_grad_(True)
+    D, bias = torch.randn(d, device=DEV).requires_grad_(True), (torch.randn(d, device=DEV) * 0.3).requires_grad_(True)
+    leaves = [u, dt, A, B, C, D, z, bias]
+    out = SS.selective_scan(u, dt, A, B, C, D, z, bias)
+    g = torch.randn(l, b, d, device=DEV).to(torch.bfloat16).transpose(0, 1) if time_major else torch.randn_like(out)
+    got = torch.autograd.grad(out, leaves, g)
+    ref_leaves = [t.detach().float().requires_grad_(True) for t in leaves]
+    ru, rdt, rA, rB, rC, rD, rz, rbias = ref_leaves
+    ref = SS.selective_scan_ref(ru, rdt, rA, rB, rC, rD, rz, rbias, True)
+    want = torch.autograd.grad(ref, ref_leaves, g.float())
+    for have, exact in zip([out, *got], [ref, *want]):
+        _close(have, exact, 4e-3 + 2e-3 * exact.abs().max().item(), rtol=4e-3)
