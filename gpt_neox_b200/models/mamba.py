@@ -11,7 +11,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops.selective_scan import causal_conv1d, selective_scan
+from ..ops.selective_scan import causal_conv1d_split, selective_scan
 from ..parallel import mappings as M
 from ..parallel import mpu
 from ..parallel.layers import ColumnParallelLinear, RowParallelLinear
@@ -67,20 +67,18 @@ class ParallelMambaBlock(nn.Module):
 
     def forward(self, hidden_states):
         seqlen, batch, _ = hidden_states.shape
+        # everything stays in the projections' [l, b, ...] order; conv and scan read it as [b, l, ...] through strides
         xz, _ = self.in_proj(hidden_states)                       # [l, b, 2*d/tp]
-        xz = xz.transpose(0, 1)                                   # [b, l, 2*d/tp]
-        x, z = xz.chunk(2, dim=-1)
-        x = causal_conv1d(x, self.conv1d.weight.squeeze(1), self.conv1d.bias, activation="silu")
-        x_dbl, _ = self.x_proj(x.reshape(batch * seqlen, -1))
+        x, z = causal_conv1d_split(xz.transpose(0, 1), self.conv1d.weight.squeeze(1), self.conv1d.bias)
+        x_dbl, _ = self.x_proj(x.transpose(0, 1).reshape(batch * seqlen, -1))
         x_dbl = M.reduce_from_model_parallel_region(x_dbl)        # dt, B, C are needed in full on every rank
-        dt, B, C = torch.split(x_dbl, [self.dt_rank, self.d_state, self.d_state], dim=-1)
-        dt = F.linear(dt, self.dt_proj.weight).view(batch, seqlen, -1)
-        B = B.reshape(batch, seqlen, self.d_state)
-        C = C.reshape(batch, seqlen, self.d_state)
+        dt, B, C = torch.split(x_dbl.view(seqlen, batch, -1).transpose(0, 1),
+                               [self.dt_rank, self.d_state, self.d_state], dim=-1)
+        dt = F.linear(dt.transpose(0, 1), self.dt_proj.weight).transpose(0, 1)
         A = -torch.exp(self.A_log.float())
-        y = selective_scan(x.contiguous(), dt, A, B, C, self.D.float(), z.contiguous(), self.dt_proj.bias.float())
-        out, _ = self.out_proj(y)
-        return out.transpose(0, 1).contiguous()
+        y = selective_scan(x, dt, A, B, C, self.D.float(), z, self.dt_proj.bias.float())
+        out, _ = self.out_proj(y.transpose(0, 1))
+        return out
 
 
 class ParallelMambaResidualLayer(nn.Module):

@@ -41,7 +41,7 @@ launch_count = 0   # number of kernel-launching library calls made by this proce
 class _CountingLib:
     """Proxy over the CDLL that counts calls into kernel launchers (``neox_*`` entry points that take a
     stream); pure queries such as ``neox_read_status`` are not counted."""
-    _NOT_LAUNCHES = {"neox_read_status", "neox_norm_bwd_blocks", "neox_sm_count_c"}
+    _NOT_LAUNCHES = {"neox_read_status", "neox_norm_bwd_blocks", "neox_sm_count_c", "neox_causal_conv_blocks"}
 
     def __init__(self, cdll):
         self._cdll = cdll

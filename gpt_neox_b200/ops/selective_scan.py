@@ -110,9 +110,72 @@ def selective_scan(u, dt, A, B, C, D, z, dt_bias):
     return selective_scan_ref(u, dt, A, B, C, D, z, dt_bias, True)
 
 
+class _CausalConv(torch.autograd.Function):
+    """``xz`` ``[b, l, d or 2 d]`` -> (activation(conv(first d channels)), the other d channels or None).  The second half is
+    a view: with it, the gradient of a projection that feeds both halves is born packed."""
+
+    @staticmethod
+    def forward(ctx, xz, weight, bias, silu):
+        b, l, _ = xz.shape
+        d = weight.shape[0]
+        w = weight.contiguous()
+        out = torch.empty(l, b, d, dtype=xz.dtype, device=xz.device).transpose(0, 1) if xz.stride(0) < xz.stride(1) \
+            else torch.empty(b, l, d, dtype=xz.dtype, device=xz.device)
+        rc = native.lib().neox_causal_conv_fwd(native.ptr(xz), native.ptr(w), native.ptr(bias), native.ptr(out),
+                                               _strides(xz, out), b, l, d, int(silu), int(xz.dtype == torch.float16),
+                                               ctypes.c_void_p(native.stream_ptr()))
+        native.check(rc, "neox_causal_conv_fwd")
+        ctx.save_for_backward(xz, w, bias)
+        ctx.silu = silu
+        return out, xz[..., d:]
+
+    @staticmethod
+    def backward(ctx, g, gz):
+        xz, w, bias = ctx.saved_tensors
+        b, l, width = xz.shape
+        d = w.shape[0]
+        g = _aligned_rows(g)
+        gxz = torch.empty(l, b, width, dtype=xz.dtype, device=xz.device).transpose(0, 1) if xz.stride(0) < xz.stride(1) \
+            else torch.empty(b, l, width, dtype=xz.dtype, device=xz.device)
+        if width > d:
+            gxz[..., d:].copy_(gz)
+        part = torch.empty(native.lib().neox_causal_conv_blocks(b, l), d, w.shape[1] + 1, dtype=torch.float32, device=xz.device)
+        rc = native.lib().neox_causal_conv_bwd(native.ptr(xz), native.ptr(w), native.ptr(bias), native.ptr(g),
+                                               native.ptr(gxz), native.ptr(part), _strides(xz, g, gxz), b, l, d,
+                                               int(ctx.silu), int(xz.dtype == torch.float16),
+                                               ctypes.c_void_p(native.stream_ptr()))
+        native.check(rc, "neox_causal_conv_bwd")
+        sums = part.sum(0).to(w.dtype)
+        return gxz, sums[:, :-1], sums[:, -1] if bias is not None else None, None
+
+
+def _aligned_rows(t):
+    """``t`` with unit channel stride and every row on a 16-byte boundary."""
+    ok = t.stride(2) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
+    return t if ok else t.contiguous()
+
+
+def _conv_kernel_ok(x, weight, bias):
+    return (x.is_cuda and native.available() and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype
+            and (bias is None or bias.dtype == x.dtype) and weight.shape[1] == 4 and weight.shape[0] % 8 == 0
+            and x.numel() > 0 and x.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
+            and x.data_ptr() % 16 == 0)
+
+
 def causal_conv1d(x, weight, bias, activation="silu"):
-    """Depth-wise causal conv over time for channel-last ``x`` ``[b, l, d]``; ``weight`` ``[d, w]``."""
+    """Depth-wise causal conv over time for channel-last ``x`` ``[b, l, d]`` (any batch and time strides); ``weight``
+    ``[d, w]``.  Width 4 in 16 bits on a GPU: one kernel with bias and SiLU (``csrc/causal_conv.cu``)."""
+    if _conv_kernel_ok(x, weight, bias):
+        return _CausalConv.apply(x, weight, bias, activation == "silu")[0]
     w = weight.shape[1]
     y = F.conv1d(x.transpose(1, 2), weight.unsqueeze(1), bias, padding=w - 1, groups=weight.shape[0])[..., : x.shape[1]]
     y = y.transpose(1, 2)
     return F.silu(y) if activation == "silu" else y
+
+
+def causal_conv1d_split(xz, weight, bias):
+    """``xz`` ``[b, l, 2 d]`` -> (``silu(conv(first half))``, second half)."""
+    if _conv_kernel_ok(xz, weight, bias):
+        return _CausalConv.apply(xz, weight, bias, True)
+    x, z = xz.chunk(2, dim=-1)
+    return causal_conv1d(x, weight, bias), z

@@ -1019,3 +1019,33 @@ def test_selective_scan_chunks_and_strides(b, l, d, time_major):
     want = torch.autograd.grad(ref, ref_leaves, g.float())
     for have, exact in zip([out, *got], [ref, *want]):
         _close(have, exact, 4e-3 + 2e-3 * exact.abs().max().item(), rtol=4e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("b,l,d,time_major,bias", [(1, 1, 8, False, True), (2, 3, 264, True, True), (3, 17, 136, True, False),
+                                                   (1, 256, 128, False, True), (2, 300, 1032, True, True)])
+def test_causal_conv_matches_fp32(b, l, d, time_major, bias, dtype):
+    """Width-4 causal convolution + SiLU of the first half of a projection, sequences shorter than the window, runs and
+    blocks part full, both orders of batch and time; forward, input, weight and bias gradients.  Outputs round once, so
+    they are within half an ulp; the weight gradient rounds once after a sum of b * l fp32 products."""
+    from gpt_neox_b200.ops import selective_scan as SS
+    torch.manual_seed(l + d)
+    xz = torch.randn(l, b, 2 * d, device=DEV).to(dtype).transpose(0, 1) if time_major else \
+        torch.randn(b, l, 2 * d, device=DEV).to(dtype)
+    xz.requires_grad_()
+    w = (torch.randn(d, 4, device=DEV) * 0.5).to(dtype).requires_grad_()
+    bs = (torch.randn(d, device=DEV) * 0.5).to(dtype).requires_grad_() if bias else None
+    assert SS._conv_kernel_ok(xz, w, bs)
+    leaves = [xz, w] + ([bs] if bias else [])
+    x, z = SS.causal_conv1d_split(xz, w, bs)
+    gx, gz = torch.randn(b, l, d, device=DEV).to(dtype), torch.randn(b, l, d, device=DEV).to(dtype)
+    got = torch.autograd.grad([x, z], leaves, [gx, gz])
+    ref = [t.detach().cpu().float().requires_grad_() for t in leaves]
+    rx, rz = SS.causal_conv1d_split(ref[0], ref[1], ref[2] if bias else None)
+    want = torch.autograd.grad([rx, rz], ref, [gx.cpu().float(), gz.cpu().float()])
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for a, b_ in zip([x, z, *got], [rx, rz, *want]):
+        _close(a.cpu(), b_, 2e-4 + ulp / 2 * b_.abs().mean().item(), rtol=ulp)
+    plain = SS.causal_conv1d(xz.detach()[..., :d], w, bs, activation=None)
+    _close(plain.cpu(), SS.causal_conv1d(xz.detach().cpu().float()[..., :d], ref[1], ref[2] if bias else None, activation=None),
+           2e-4 + ulp / 2, rtol=ulp)
