@@ -1049,3 +1049,31 @@ def test_causal_conv_matches_fp32(b, l, d, time_major, bias, dtype):
     plain = SS.causal_conv1d(xz.detach()[..., :d], w, bs, activation=None)
     _close(plain.cpu(), SS.causal_conv1d(xz.detach().cpu().float()[..., :d], ref[1], ref[2] if bias else None, activation=None),
            2e-4 + ulp / 2, rtol=ulp)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (1, 2048, 4096), (3, 24, 72), (8, 1000, 1032), (9, 16, 64), (16, 4104, 520),
+                                   (17, 40, 2056), (32, 264, 136), (33, 64, 128)])
+def test_few_row_gemm_matches_fp32(M, N, K, dtype):
+    """The weight-streaming kernel (up to 32 rows; 33 takes the tile kernel): part-filled row groups, weight tiles and
+    k-blocks, one k-block and K split over a cluster, all epilogues.  The 16-bit result is within half an ulp of the fp32
+    value, whose own summation error is below K * 2^-24 of the sum of magnitudes."""
+    from gpt_neox_b200.ops import gemm as G
+    torch.manual_seed(M * N + K)
+    x = torch.randn(M, K + 8, device=DEV).to(dtype)[:, :K]
+    w, bias, add = torch.randn(N, K, device=DEV).to(dtype), torch.randn(N, device=DEV).to(dtype), torch.randn(M, N, device=DEV)
+    aux, scale = torch.randn(M, N, device=DEV).to(dtype), K ** -0.5
+    assert G.use_skinny_kernel(M, N, K, False, False) == (M <= 32)
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+
+    def check(**kw):
+        got, want = G.gemm(x, w, alpha=scale, **kw), G.gemm_ref(x, w, alpha=scale, **{"out_dtype": dtype, **kw})
+        for a, b in zip(got, want) if kw.get("want_preact") else [(got, want)]:
+            _close(a, b, 1e-4 if kw.get("out_dtype") == torch.float32 else half_ulp / 8,
+                   rtol=1e-4 if kw.get("out_dtype") == torch.float32 else 2 * half_ulp)
+    check()
+    check(bias=bias, add=add.to(dtype))
+    check(bias=bias, act=G.ACT_GELU, want_preact=True)
+    check(act=G.ACT_DGELU, aux=aux)
+    check(out_dtype=torch.float32, add=add)
+    assert torch.equal(G.gemm(x, w, bias=bias), G.gemm(x, w, bias=bias))       # fixed summation order
