@@ -22,7 +22,8 @@ import torch.nn.functional as F
 
 from ..ops import functional as OF
 from ..ops.sparse_attention import block_sparse_attention
-from ..ops.attention import flash_attention, packed_qkv_attention, packed_qkv_ok
+from ..ops.attention import (decode_attention, decode_attention_ok, flash_attention, packed_qkv_attention,
+                             packed_qkv_ok)
 from ..ops.linear import dead_outputs, linear as fused_linear
 from ..parallel import mappings as M
 from ..parallel import mpu
@@ -329,6 +330,26 @@ class ParallelSelfAttention(nn.Module):
         probs = torch.softmax(scores.masked_fill(future, float("-inf")), dim=-1).to(q.dtype)
         return torch.einsum("bhqk,kbhd->qbhd", probs, vals)
 
+    def _decode_step(self, q, k, v, layer_past, static_step):
+        """One new token against the cache in one launch (rotary embedding, append, attention): ``(context, present)``, or
+        ``None`` where that kernel does not apply."""
+        if self.rpe is not None or self.sparse or (self.dropout_p > 0 and self.training) or not decode_attention_ok(q, k, v):
+            return None
+        if static_step:
+            cache, n, pos, present = self.static_kv, self.static_kv.shape[1] - 1, self.static_pos, self.static_kv
+            if cache.dtype != k.dtype:
+                return None
+        else:
+            present = _reserve_kv_rows(layer_past, k)
+            cache, n, pos = present._kv_buf, present.shape[1] - 1, None
+        cos = sin = None
+        if self.rotary_emb is not None:
+            cos, sin = self.rotary_emb(v, seq_len=n + 1)
+        slopes = self.alibi_embed.slopes if self.pos_emb == "alibi" else None
+        ctx = decode_attention(q, k, v, cache, n, pos, cos, sin, softmax_scale=(self.coeff or 1.0) / self.norm_factor,
+                               window=self.sliding_window_width, alibi_slopes=slopes)
+        return ctx, present
+
     def _packed_path(self, hidden_states, layer_past):
         """rotary + flash attention on the packed QKV projection, in place (training / no kv-cache)."""
         if self.gqa or self.use_qk_layernorm or self.use_cache or self.rpe is not None or self.sparse or \
@@ -362,6 +383,14 @@ class ParallelSelfAttention(nn.Module):
         if self.use_qk_layernorm:
             q, k = self.qk_layernorm(q), self.qk_layernorm(k)
         static_step = self.static_kv is not None and self.use_cache and k.shape[0] == 1 and self.static_filled
+        if static_step or (self.use_cache and self.static_kv is None and k.shape[0] == 1 and layer_past is not None
+                           and layer_past[0].numel() > 0):
+            step = self._decode_step(q, k, v, layer_past, static_step)
+            if step is not None:
+                ctx, present = step
+                ctx = ctx.reshape(1, ctx.shape[1], self.hidden_size_per_partition)
+                out, bias = self.dense(ctx, residual=residual, fuse_bias=fuse_bias)
+                return [out, present], bias
         if self.rotary_emb is not None and static_step:
             # decoding against the fixed-capacity cache: the position lives on the device (``static_pos``), so the
             # same launch sequence serves every step and can be replayed from a CUDA graph
@@ -431,9 +460,9 @@ def _zero_scalar(device, dtype):
     return z
 
 
-def _extend_kv_cache(layer_past, k, v):
-    """``[2, n + s, b, heads, d]`` view holding the cached keys / values followed by the new ones.  The view carries
-    its backing buffer (``_kv_buf``, capacity grown geometrically), so the next step appends in place when there is
+def _reserve_kv_rows(layer_past, k):
+    """``[2, n + s, b, heads, d]`` view holding the cached keys / values followed by room for the ``s`` rows of ``k``.  The
+    view carries its backing buffer (``_kv_buf``, capacity grown geometrically), so the next step appends in place when there is
     room: O(s) per step instead of the O(n) of concatenating (reference: ``torch.cat`` + ``torch.stack`` per step,
     ``megatron/model/transformer.py:1003-1012``)."""
     s = k.shape[0]
@@ -450,11 +479,18 @@ def _extend_kv_cache(layer_past, k, v):
             new[0, :n].copy_(layer_past[0])
             new[1, :n].copy_(layer_past[1])
         buf = new
-    buf[0, n:n + s].copy_(k)
-    buf[1, n:n + s].copy_(v)
     buf._filled = n + s
     present = buf[:, :n + s]
     present._kv_buf = buf
+    return present
+
+
+def _extend_kv_cache(layer_past, k, v):
+    """The cached keys / values followed by the new ones (see ``_reserve_kv_rows``)."""
+    present = _reserve_kv_rows(layer_past, k)
+    s = k.shape[0]
+    present[0, -s:].copy_(k)
+    present[1, -s:].copy_(v)
     return present
 
 

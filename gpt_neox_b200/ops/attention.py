@@ -231,3 +231,40 @@ def flash_attention(q, k, v, causal=True, softmax_scale=None, window=None, alibi
         slopes = alibi_slopes.float().contiguous() if alibi_slopes is not None else None
         return _FlashFn.apply(q, k, v, causal, scale, window, slopes)
     return attention_ref(q, k, v, causal, scale, window, alibi_slopes, bias)
+
+
+# ------------------------------------------------------------------------------------ one new token against the cache
+def decode_attention_ok(q, k, v) -> bool:
+    """Can ``decode_attention`` take these projections ([1, b, heads, d], before the rotary embedding)?"""
+    return (q.is_cuda and native.available() and q.dtype in (torch.bfloat16, torch.float16) and k.dtype == q.dtype
+            and v.dtype == q.dtype and q.shape[0] == 1 and k.shape[0] == 1 and q.shape[-1] in (64, 96, 128)
+            and q.stride(-1) == 1 and k.stride(-1) == 1 and v.stride(-1) == 1 and q.shape[2] % k.shape[2] == 0
+            and not (torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad)))
+
+
+def decode_attention(q, k, v, cache, n, pos=None, cos=None, sin=None, softmax_scale=None, window=None, alibi_slopes=None):
+    """Rotary embedding of one new token, append of its key / value to ``cache`` and attention over everything cached:
+    one launch (``csrc/decode_attn.cu``).
+
+    ``cache``: contiguous ``[2, capacity, b, heads_kv, d]``.  The new token is row ``n`` of it (``n`` rows are filled), or,
+    with ``pos`` (one int64 on the device), row ``pos`` with ``n`` an upper bound.  ``cos`` / ``sin``: the whole rotary
+    tables ``[rows, 1, 1, rot]``.  Returns ``[1, b, heads_q, d]``."""
+    _, b, hq, d = q.shape
+    hkv = k.shape[2]
+    assert cache.is_contiguous() and cache.dtype == q.dtype and cache.shape[2:] == (b, hkv, d) and 0 <= n < cache.shape[1]
+    scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(d)
+    flop_count.attention(b, hq, 1, n + 1, d, True)
+    rot = 0
+    if cos is not None:
+        rot = cos.shape[-1]
+        cos, sin = cos.float().contiguous(), sin.float().contiguous()
+        assert cos.numel() // rot > n
+    slopes = alibi_slopes.float().contiguous() if alibi_slopes is not None else None
+    out = torch.empty(1, b, hq, d, dtype=q.dtype, device=q.device)
+    strides = (ctypes.c_longlong * 6)(q.stride(1), q.stride(2), k.stride(1), k.stride(2), v.stride(1), v.stride(2))
+    rc = native.lib().neox_decode_attn(
+        native.ptr(q), native.ptr(k), native.ptr(v), native.ptr(out), native.ptr(cache[0]), native.ptr(cache[1]),
+        native.ptr(cos), native.ptr(sin), native.ptr(pos), native.ptr(slopes), strides, n, cache.shape[1], b, hq, hkv, d,
+        rot, int(window if window is not None else -1), ctypes.c_float(scale), int(q.dtype == torch.float16), _s())
+    native.check(rc, "neox_decode_attn")
+    return out

@@ -1077,3 +1077,40 @@ def test_few_row_gemm_matches_fp32(M, N, K, dtype):
     check(act=G.ACT_DGELU, aux=aux)
     check(out_dtype=torch.float32, add=add)
     assert torch.equal(G.gemm(x, w, bias=bias), G.gemm(x, w, bias=bias))       # fixed summation order
+
+
+@pytest.mark.parametrize("n,b,hq,hkv,d,rot,window,alibi,dtype", [
+    (1, 1, 4, 4, 64, 16, None, False, torch.float16), (31, 2, 4, 1, 128, 128, None, False, torch.bfloat16),
+    (129, 1, 4, 2, 96, 24, None, True, torch.bfloat16), (700, 2, 8, 8, 64, 64, None, False, torch.bfloat16),
+    (700, 1, 4, 4, 128, 32, 37, False, torch.float16), (2047, 1, 2, 2, 128, 0, 1500, True, torch.bfloat16),
+    (300, 20, 16, 16, 64, 16, 0, False, torch.bfloat16)])
+def test_decode_attention_matches_rotary_append_and_attention(n, b, hq, hkv, d, rot, window, alibi, dtype):
+    """One launch against the separate steps in fp32: rotary embedding, append, softmax over the cache (split over one
+    to eight CTAs), grouped queries, window, ALiBi, packed strided projections, position on the host and on the device.
+    The output is a convex combination of values, so its error is that of 16-bit weights' fp32 sums plus half an ulp."""
+    from gpt_neox_b200.models.positional import RotaryEmbedding
+    from gpt_neox_b200.ops import attention as A
+    from gpt_neox_b200.ops import functional as OF
+    torch.manual_seed(n + d)
+    packed = torch.randn(1, b, hq + 2 * hkv, d, device=DEV).to(dtype)
+    q, k, v = packed.split([hq, hkv, hkv], dim=2)
+    cap = n + 1 if n == 2047 else n + 9
+    cache = torch.randn(2, cap, b, hkv, d, device=DEV).to(dtype)
+    cos = sin = None
+    kr, qr = k, q
+    if rot:
+        cos, sin = RotaryEmbedding(rot, cap).to(DEV)(q, seq_len=cap)
+        qr, kr = OF.rope_ref(q, cos[n:n + 1], sin[n:n + 1]), OF.rope_ref(k, cos[n:n + 1], sin[n:n + 1])
+    slopes = torch.rand(hq, device=DEV) if alibi else None
+    keys = torch.cat([cache[0, :n], kr]).float()
+    vals = torch.cat([cache[1, :n], v]).float()
+    want = A.attention_ref(qr.float(), keys, vals, True, 0.1, window, slopes)
+    assert A.decode_attention_ok(q, k, v)
+    for pos in (None, torch.tensor([n], device=DEV)):
+        c = cache.clone()
+        got = A.decode_attention(q, k, v, c, n if pos is None else cap - 1, pos, cos, sin, 0.1, window, slopes)
+        _close(got, want, 1e-3, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10)
+        _close(c[0, n], kr[0], 1e-3, rtol=2.0 ** -8)                   # the rotated key, to the rounding of its 16 bits
+        assert torch.equal(c[1, n], v[0])
+        keep = torch.arange(cap, device=DEV) != n
+        assert torch.equal(c[:, keep], cache[:, keep])
