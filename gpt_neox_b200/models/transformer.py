@@ -552,7 +552,7 @@ class ParallelTransformerLayer(nn.Module):
                 x2 = x1
             else:
                 x1, x2, residual = OF.norm_fan_out(x, [self.input_layernorm, self.post_attention_layernorm])
-            if fuse and self.mlp_type == "regular" and not self.use_cache:
+            if fuse and self.mlp_type == "regular":
                 # attention partial (+ its bias) [+ residual when no reduction follows] accumulated by the
                 # GEMM epilogues:  out = residual + attn + b_a + mlp + b_m
                 attn_res = residual if self.tp == 1 else None
@@ -563,6 +563,8 @@ class ParallelTransformerLayer(nn.Module):
                 # the attention output bias rides in the dense GEMM's epilogue (every rank adds its own to its partial)
                 a_out, a_bias = self.attention(x1, attention_mask, layer_past=layer_past, residual=attn_res,
                                                fuse_bias=True, dead_dense=dead)
+                if self.use_cache:
+                    a_out, self.layer_past = a_out
                 if a_bias is not None:
                     a_out = a_out + a_bias
                 if self.tp == 1:
@@ -588,25 +590,21 @@ class ParallelTransformerLayer(nn.Module):
 
         # sequential residual
         h1, residual = OF.norm_fan_out(x, [self.input_layernorm])
-        can_fuse_res = fuse and not self.use_cache
-        a_out, a_bias = self.attention(h1, attention_mask, layer_past=layer_past,
-                                       residual=residual if (can_fuse_res and self.attention.dense.bias is None) else None)
+        # without dropout, bias and residual ride in the output projections' epilogues (after the reduction, if there is one)
+        a_out, a_bias = self.attention(h1, attention_mask, layer_past=layer_past, residual=residual if fuse else None,
+                                       fuse_bias=fuse)
         if self.use_cache:
-            a_out, presents = a_out
-            self.layer_past = presents
-        if can_fuse_res and self.attention.dense.bias is None:
-            x = a_out
-        else:
-            x = OF.bias_dropout_add(a_out, a_bias, residual, p, self.training)
+            a_out, self.layer_past = a_out
+        x = a_out if fuse else OF.bias_dropout_add(a_out, a_bias, residual, p, self.training)
         ln2, x = OF.norm_fan_out(x, [self.post_attention_layernorm])
         if self.mlp_type == "moe":
             m_out, moe_loss = self.mlp(ln2)
             out = OF.bias_dropout_add(m_out, None, x, p, self.training)
         else:
-            fuse_m = can_fuse_res and self.mlp.linear2.bias is None
             # (see the parallel-residual branch: in a recomputed block tail only linear2's inputs are needed)
-            m_out, m_bias = self.mlp(ln2, residual=x if fuse_m else None, dead_output=fuse_m and recompute_tail())
-            out = m_out if fuse_m else OF.bias_dropout_add(m_out, m_bias, x, p, self.training)
+            m_out, m_bias = self.mlp(ln2, residual=x if fuse else None, fuse_bias=fuse,
+                                     dead_output=fuse and recompute_tail())
+            out = m_out if fuse else OF.bias_dropout_add(m_out, m_bias, x, p, self.training)
         return out, moe_loss
 
 
