@@ -347,6 +347,66 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, 
 
 // In-place rotary embedding of the first `rot` dims of every head of q and k (views of one packed QKV tensor): one
 // thread owns the pair (e, e + rot/2), so nothing is read after it was overwritten.  cs / sn: [s, rot] fp32.
+// The same rotation, VEC elements of each half per access.  Bound by the bytes of the rotated parts, read and written in
+// place.  One element per thread, the general form below, made it 16-bit accesses and 64-bit divisions: 38.7 us for 8192
+// tokens x 24 heads of 64, whole heads rotated (8 us of bytes), 117 us for 8192 x 128 heads of 96, 24 rotated.  A thread
+// keeps its piece of the fp32 tables, which is twice the size of the elements it rotates, for ROPE_HEADS heads.
+// The two shapes take 13.8 and 53.8 us here.
+constexpr int ROPE_HEADS = 4;
+template <typename T, int VEC>
+__global__ void __launch_bounds__(256) rope_qk_inplace_vec_kernel(T* __restrict__ q, T* __restrict__ k,
+                                                                  const float* __restrict__ cs,
+                                                                  const float* __restrict__ sn, int s, int b, int hq, int hk,
+                                                                  int rot, long long q_ss, long long q_sb, long long q_sh,
+                                                                  long long k_ss, long long k_sb, long long k_sh,
+                                                                  int inverse) {
+    struct alignas(VEC * 2) Pack {
+        T v[VEC];
+    };
+    const int half = rot >> 1, nv = half / VEC, heads = hq + hk, groups = (heads + ROPE_HEADS - 1) / ROPE_HEADS;
+    const long long item = blockIdx.x * 256ll + threadIdx.x;
+    const long long token = item / (nv * groups);
+    const int in_token = (int)(item - token * (nv * groups));
+    if (token >= (long long)s * b) return;
+    const int e = in_token % nv * VEC, h0 = in_token / nv * ROPE_HEADS;
+    const int sI = (int)(token / b), bb = (int)(token - (long long)sI * b);
+    T* xp[ROPE_HEADS];
+    Pack lo[ROPE_HEADS], hi[ROPE_HEADS];
+#pragma unroll
+    for (int i = 0; i < ROPE_HEADS; ++i) {
+        const int hh = h0 + i;
+        if (hh < heads) {
+            xp[i] = (hh < hq ? q + sI * q_ss + bb * q_sb + hh * q_sh : k + sI * k_ss + bb * k_sb + (hh - hq) * k_sh) + e;
+            lo[i] = *reinterpret_cast<const Pack*>(xp[i]);
+            hi[i] = *reinterpret_cast<const Pack*>(xp[i] + half);
+        }
+    }
+    const float* cr = cs + (long long)sI * rot + e;
+    const float* sr = sn + (long long)sI * rot + e;
+    const float sg = inverse ? -1.f : 1.f;
+    float c0[VEC], c1[VEC], s0[VEC], s1[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+        c0[j] = __ldg(cr + j);
+        c1[j] = __ldg(cr + half + j);
+        s0[j] = __ldg(sr + j) * sg;
+        s1[j] = __ldg(sr + half + j) * sg;
+    }
+#pragma unroll
+    for (int i = 0; i < ROPE_HEADS; ++i) {
+        if (h0 + i < heads) {
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) {
+                const float a = to_f<T>(lo[i].v[j]), c2 = to_f<T>(hi[i].v[j]);
+                lo[i].v[j] = from_f<T>(a * c0[j] - c2 * s0[j]);
+                hi[i].v[j] = from_f<T>(c2 * c1[j] + a * s1[j]);
+            }
+            *reinterpret_cast<Pack*>(xp[i]) = lo[i];
+            *reinterpret_cast<Pack*>(xp[i] + half) = hi[i];
+        }
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) rope_qk_inplace_kernel(T* __restrict__ q, T* __restrict__ k,
                                                               const float* __restrict__ cs, const float* __restrict__ sn,
@@ -833,6 +893,30 @@ int neox_rope_qk_inplace(void* q, void* k, const float* cs, const float* sn, int
     if (total <= 0) return 0;
     if (rot % 2) return NEOX_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
+    // Vectors of 8 or 4 elements where every vector of both halves of every head starts on a multiple of its size.
+    const int half = rot / 2;
+    const long long strides = q_ss | q_sb | q_sh | k_ss | k_sb | k_sh;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k);
+    auto fits = [&](int vec) { return half % vec == 0 && strides % vec == 0 && base % (vec * 2) == 0; };
+    const int vec = dtype == 1 ? 0 : fits(8) ? 8 : fits(4) ? 4 : 0;
+    if (vec) {
+        const long long items = (long long)s * b * (half / vec) * ((hq + hk + ROPE_HEADS - 1) / ROPE_HEADS);
+        const long long blocks = (items + 255) / 256;
+        if (blocks <= 0x7fffffff) {
+#define ROPE_VEC(T, V)                                                                                                   \
+    rope_qk_inplace_vec_kernel<T, V><<<(int)blocks, 256, 0, st>>>((T*)q, (T*)k, cs, sn, s, b, hq, hk, rot, q_ss, q_sb, q_sh, \
+                                                                  k_ss, k_sb, k_sh, inverse)
+            if (dtype == 0) {
+                if (vec == 8) ROPE_VEC(__nv_bfloat16, 8);
+                else ROPE_VEC(__nv_bfloat16, 4);
+            } else {
+                if (vec == 8) ROPE_VEC(__half, 8);
+                else ROPE_VEC(__half, 4);
+            }
+#undef ROPE_VEC
+            return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
+        }
+    }
     DISPATCH(dtype, (rope_qk_inplace_kernel<T><<<grid_for(total, 16), 256, 0, st>>>(
                         (T*)q, (T*)k, cs, sn, s, b, hq, hk, rot, q_ss, q_sb, q_sh, k_ss, k_sb, k_sh, inverse)));
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
