@@ -590,24 +590,58 @@ __global__ void __launch_bounds__(256) ce_bwd_bf16_kernel(const __nv_bfloat16* _
 }
 
 // ------------------------------------------------------------------ optimizers
-template <typename OUT>
+// Adam over a flat shard, in place.  Bound by bytes: four fp32 streams in, three out and the 16-bit copy, 30 per element.
+// VEC = 4: one 16-byte access per stream and thread, without keeping any of it in the caches; with 4-byte accesses the
+// same pass ran at 4.8 TB/s over 1.5e9 elements and 5.4 TB/s over 0.7e9 and now at 5.4 and 5.7 TB/s.
+template <typename OUT, int VEC>
 __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                                                    const float* __restrict__ g, OUT* __restrict__ out, long long n,
                                                    float lr, float b1, float b2, float eps, float wd, float bc1,
                                                    float bc2, float gs, int adamw) {
     const float step = lr / bc1;
     const float isb2 = rsqrtf(bc2);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float gi = g[i] * gs;
-        float pi = p[i];
+    auto update = [&](float gi, float& pi, float& mi, float& vi) {
+        gi *= gs;
         if (!adamw && wd != 0.f) gi += wd * pi;
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
+        mi = b1 * mi + (1.f - b1) * gi;
+        vi = b2 * vi + (1.f - b2) * gi * gi;
         float upd = step * (mi / (sqrtf(vi) * isb2 + eps));
         if (adamw && wd != 0.f) upd += lr * wd * pi;
         pi -= upd;
+    };
+    const long long nvec = VEC == 4 ? n / 4 : 0, first = blockIdx.x * (long long)blockDim.x + threadIdx.x,
+                    stride = (long long)gridDim.x * blockDim.x;
+    if constexpr (VEC == 4) {
+        struct alignas(sizeof(OUT) * 4) Pack {
+            OUT v[4];
+        };
+        for (long long i = first; i < nvec; i += stride) {
+            const float4 gv = __ldcs(reinterpret_cast<const float4*>(g) + i);
+            float4 pv = __ldcs(reinterpret_cast<const float4*>(p) + i);
+            float4 mv = __ldcs(reinterpret_cast<const float4*>(m) + i);
+            float4 vv = __ldcs(reinterpret_cast<const float4*>(v) + i);
+            update(gv.x, pv.x, mv.x, vv.x);
+            update(gv.y, pv.y, mv.y, vv.y);
+            update(gv.z, pv.z, mv.z, vv.z);
+            update(gv.w, pv.w, mv.w, vv.w);
+            __stcs(reinterpret_cast<float4*>(m) + i, mv);
+            __stcs(reinterpret_cast<float4*>(v) + i, vv);
+            __stcs(reinterpret_cast<float4*>(p) + i, pv);
+            if (out) {
+                Pack o;
+                o.v[0] = from_f<OUT>(pv.x);
+                o.v[1] = from_f<OUT>(pv.y);
+                o.v[2] = from_f<OUT>(pv.z);
+                o.v[3] = from_f<OUT>(pv.w);
+                reinterpret_cast<Pack*>(out)[i] = o;
+            }
+        }
+    }
+    for (long long i = nvec * VEC + first; i < n; i += stride) {
+        float pi = p[i], mi = m[i], vi = v[i];
+        update(g[i], pi, mi, vi);
+        m[i] = mi;
+        v[i] = vi;
         p[i] = pi;
         if (out) out[i] = from_f<OUT>(pi);
     }
@@ -962,14 +996,25 @@ int neox_adam_step(float* p, float* m, float* v, const float* g, void* out, int 
                    float b1, float b2, float eps, float wd, float bc1, float bc2, float gs, int adamw, void* stream) {
     if (n <= 0) return 0;
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = grid_for(n, 16);
-    if (!out || out_dtype == 1)
-        adam_kernel<float><<<grid, 256, 0, st>>>(p, m, v, g, (float*)out, n, lr, b1, b2, eps, wd, bc1, bc2, gs, adamw);
-    else if (out_dtype == 0)
-        adam_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, m, v, g, (__nv_bfloat16*)out, n, lr, b1, b2, eps, wd, bc1,
-                                                          bc2, gs, adamw);
-    else
-        adam_kernel<__half><<<grid, 256, 0, st>>>(p, m, v, g, (__half*)out, n, lr, b1, b2, eps, wd, bc1, bc2, gs, adamw);
+    auto aligned = [](const void* q, int bytes) { return (reinterpret_cast<uintptr_t>(q) & (bytes - 1)) == 0; };
+    // a shard may start anywhere in a flat buffer: four elements at a time only where all of its tensors allow it
+    const bool vec = aligned(p, 16) && aligned(m, 16) && aligned(v, 16) && aligned(g, 16) &&
+                     (!out || aligned(out, out_dtype == 1 ? 16 : 8));
+    const int grid = grid_for(vec ? (n + 3) / 4 : n, vec ? 8 : 16);
+#define ADAM(T, VEC) \
+    adam_kernel<T, VEC><<<grid, 256, 0, st>>>(p, m, v, g, (T*)out, n, lr, b1, b2, eps, wd, bc1, bc2, gs, adamw)
+#define ADAM_T(T) \
+    if (vec) ADAM(T, 4); \
+    else ADAM(T, 1)
+    if (!out || out_dtype == 1) {
+        ADAM_T(float);
+    } else if (out_dtype == 0) {
+        ADAM_T(__nv_bfloat16);
+    } else {
+        ADAM_T(__half);
+    }
+#undef ADAM_T
+#undef ADAM
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 // qm / qv hold ceil(n / 256) * 256 quantised states, sm / sv one fp32 scale per block of 256.
