@@ -69,7 +69,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 
     const int num_m = (p.M + BM - 1) / BM;
     const int num_n = (p.N + BN - 1) / BN;
-    const int ntiles = p.group_mode ? __ldg(p.group_ntiles) : num_m * num_n;
+    const int ntiles = p.group_mode ? __ldg(p.group_ntiles) : num_m * num_n * p.splits;
     const int nk = (p.K + BK - 1) / BK;
 
     if (warp == 0) {
@@ -90,7 +90,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                     uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
                     uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
                     if (!p.a_mn) {
-                        tma_load_2d(a_dst, &tmA, &full[stage], kb * BK, t.a_m0);
+                        tma_load_2d(a_dst, &tmA, &full[stage], t.a_k0 + kb * BK, t.a_m0);
                     } else {
 #pragma unroll
                         for (int j = 0; j < BM / 64; ++j)
@@ -98,7 +98,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                                         t.a_k0 + kb * BK);
                     }
                     if (!p.b_mn) {
-                        tma_load_2d(b_dst, &tmB, &full[stage], kb * BK, t.b_n0);
+                        tma_load_2d(b_dst, &tmB, &full[stage], t.b_k0 + kb * BK, t.b_n0);
                     } else {
 #pragma unroll
                         for (int j = 0; j < BN / 64; ++j)
@@ -137,7 +137,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                 }
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * BN;
-                const int nk_t = p.group_mode == 2 ? __ldg(p.groups + tile).y : nk;
+                const int nk_t = tile_info(p, tile, num_m, num_n, nk).nk;
                 for (int kb = 0; kb < nk_t; ++kb) {
                     if (!mbar_wait(&full[stage], phase)) {
                         atomicExch(p.status, 103);
@@ -336,6 +336,25 @@ extern "C" int neox_gemm_bf16_rowmap(const void* A, const void* B, void* D, int 
                         aux, ldaux, act, alpha, row_ptrs, 0, stream_);
 }
 
+// Contraction splits of an accumulating product.  Weight gradients of narrow models have few output tiles and a long
+// contraction (all tokens): 768 x 768 over 8192 tokens is 18 tiles, each walking 128 k-blocks while 130 SMs idle.  The
+// cost of a choice is rounds of tiles x blocks per tile; splits are taken while they cut that by an eighth and leave a
+// tile 8 k-blocks, below which filling the pipeline and the epilogue's atomic pass over the tile outweigh the product.
+// Mean over a 125M model's four weight gradients (8192 tokens) 56.6 -> 35.4 us, a Mamba-130M's 41.9 -> 24.9 us.  The order
+// of the additions to an element is not fixed.
+static int pick_splits(long long tiles, int nk, int sms) {
+    int best = 1;
+    double cost = (double)((tiles + sms - 1) / sms) * nk;
+    for (int s = 2; s <= 8 && nk / s >= 8; ++s) {
+        const double c = (double)((tiles * s + sms - 1) / sms) * ((nk + s - 1) / s);
+        if (c < cost * 0.875) {
+            best = s;
+            cost = c;
+        }
+    }
+    return best;
+}
+
 // The general entry point: h16 = 0 for bf16, 1 for fp16 (operands and every 16-bit epilogue tensor share the type).
 extern "C" int neox_gemm_16(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb,
                             long long ldd, int a_mn, int b_mn, int d_fp32, const void* bias, const void* add,
@@ -387,10 +406,12 @@ extern "C" int neox_gemm_16(const void* A, const void* B, void* D, int M, int N,
         attr_set = true;
     }
     const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
-    int grid = num_m * num_n;
     const int sms = neox_sm_count();
+    const bool inplace = d_fp32 && add_fp32 && add == D && ldadd == ldd && !preact && act == 0 && !bias;
+    if (inplace) p.splits = pick_splits((long long)num_m * num_n, (K + BK - 1) / BK, sms);
+    long long grid = (long long)num_m * num_n * p.splits;
     if (grid > sms) grid = sms;
-    gemm_bf16_tcgen05_kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+    gemm_bf16_tcgen05_kernel<<<(int)grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
