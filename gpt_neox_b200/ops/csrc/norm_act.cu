@@ -1,5 +1,5 @@
 // Bandwidth-bound row kernels: LayerNorm / RMSNorm forward+backward and the fused bias / activation /
-// residual element-wise ops.  One CTA per row (grid-stride over rows), 16-byte vector accesses, the
+// residual element-wise ops.  One warp or CTA per row (grid-stride over rows), 16-byte vector accesses, the
 // row is held in registers between the statistics pass and the normalisation pass so every input
 // byte is read from HBM exactly once.  fp32 statistics for all storage dtypes (bf16 / fp16 / fp32).
 //
@@ -11,9 +11,9 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
-namespace {
+#include <type_traits>
 
-constexpr int MAXV = 4;  // vectors of 8 elements cached per thread
+namespace {
 
 template <typename T>
 struct Vec8;
@@ -109,104 +109,110 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// Sum over the CTA; every thread receives the result.  `red` is a 33-float shared scratch.
-__device__ __forceinline__ float block_sum(float v, float* red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+// Sums over the CTA; every thread receives the result.  One barrier: callers alternate between two buffers, so that a
+// buffer is written again only after a barrier that follows its last read.
+__device__ __forceinline__ float block_sum(float v, float (&red)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     v = warp_sum(v);
-    __syncthreads();
     if (lane == 0) red[warp] = v;
     __syncthreads();
-    float t = (threadIdx.x < nw) ? red[threadIdx.x] : 0.f;
-    if (warp == 0) {
-        t = warp_sum(t);
-        if (lane == 0) red[32] = t;
-    }
-    __syncthreads();
-    return red[32];
+    float t = 0.f;
+    for (int w = 0; w < nw; ++w) t += red[w];
+    return t;
 }
 
-__device__ __forceinline__ void block_sum2(float& a, float& b, float* red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+__device__ __forceinline__ void block_sum2(float& a, float& b, float2 (&red)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     a = warp_sum(a);
     b = warp_sum(b);
+    if (lane == 0) red[warp] = make_float2(a, b);
     __syncthreads();
-    if (lane == 0) {
-        red[warp] = a;
-        red[33 + warp] = b;
+    a = b = 0.f;
+    for (int w = 0; w < nw; ++w) {
+        const float2 t = red[w];
+        a += t.x;
+        b += t.y;
     }
-    __syncthreads();
-    float ta = (threadIdx.x < nw) ? red[threadIdx.x] : 0.f;
-    float tb = (threadIdx.x < nw) ? red[33 + threadIdx.x] : 0.f;
-    if (warp == 0) {
-        ta = warp_sum(ta);
-        tb = warp_sum(tb);
-        if (lane == 0) {
-            red[32] = ta;
-            red[65] = tb;
-        }
-    }
-    __syncthreads();
-    a = red[32];
-    b = red[65];
 }
 
-// ------------------------------------------------------------------ LayerNorm
+// ------------------------------------------------------------------ LayerNorm / RMSNorm
 // RMS == false: y = (x - mean) * rstd * gamma + beta,   stat0 = mean, stat1 = rstd
 // RMS == true : y = x * rinv * gamma + beta with rinv = 1 / (sqrt(mean(x^2)) + eps),  stat1 = rinv
-template <typename T, bool RMS>
-__global__ void __launch_bounds__(256) norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma,
-                                                       const T* __restrict__ beta, T* __restrict__ y,
-                                                       float* __restrict__ stat0, float* __restrict__ stat1,
-                                                       int rows, int cols, float eps) {
-    __shared__ float red[66];
+//
+// Bound by bytes: x in, y out (backward: x, g, the addend in, dx out).  What keeps a row kernel from them is the serial
+// chain of a row (load, one or two reductions, store), so rows must overlap: rows of up to 1024 columns belong to one
+// warp each (no barrier at all, 16 to 32 rows in flight on an SM), longer rows to a CTA with one barrier per reduction.
+// V, the vectors of 8 elements a thread holds, is a template parameter so that a thread keeps registers only for what it
+// has; with room for 4 compiled in throughout, 768-column rows ran at 18 % of the copy bandwidth backward and 20 % forward.
+// In both forms the next row is requested before this row's reductions.  8192 rows, before and now: 768 columns forward
+// 19.0 -> 8.0 us, backward with addend 44.1 -> 15.4 (7.6 of bytes); 6144 columns 83 -> 55 and 223 -> 157 (60 of bytes);
+// 4096, RMS 42 -> 24 and 158 -> 104; 5781 rows of 1024 in fp16 14.5 -> 8.3 and 30.3 -> 13.5.
+constexpr int ROW_WARPS = 8;          // rows of up to 1024 columns: warps (rows) per CTA
+constexpr int ROW_COLS = 1024;
+constexpr int CTA_THREADS = 384;      // longer rows: V = ceil(vectors / 384), 1 to 3; V = 0 re-reads the row instead
+
+// Sum over whoever holds the row: a warp or the CTA.
+template <bool WARP>
+__device__ __forceinline__ float row_sum(float v, float (&red)[32]) {
+    if constexpr (WARP) return warp_sum(v);
+    else return block_sum(v, red);
+}
+
+template <typename T, bool RMS, int V, bool WARP>
+__global__ void __launch_bounds__(WARP ? ROW_WARPS * 32 : CTA_THREADS)
+norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
+                float* __restrict__ stat0, float* __restrict__ stat1, int rows, int cols, float eps) {
+    __shared__ float red0[32], red1[32];
+    constexpr bool CACHED = V > 0;
     const int nvec = cols >> 3;
-    const bool cached = nvec <= MAXV * (int)blockDim.x;
-    // Cached path: the next row's (packed) data is requested before this row's reductions start, so two rows per
-    // CTA are in flight and the loads overlap the block-wide sums.
-    typename Vec8<T>::Raw nxt[MAXV];
+    const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, width = WARP ? 32 : blockDim.x;
+    const int first = WARP ? blockIdx.x * ROW_WARPS + (threadIdx.x >> 5) : blockIdx.x;
+    const int step = WARP ? gridDim.x * ROW_WARPS : gridDim.x;
+    typename Vec8<T>::Raw nxt[CACHED ? V : 1];
     auto fetch = [&](int r) {
 #pragma unroll
-        for (int j = 0; j < MAXV; ++j) {
-            const int c = threadIdx.x + j * blockDim.x;
+        for (int j = 0; j < V; ++j) {
+            const int c = tid + j * width;
             if (c < nvec) nxt[j] = Vec8<T>::raw_load(x + (size_t)r * cols + c * 8);
         }
     };
-    if (cached && (int)blockIdx.x < rows) fetch(blockIdx.x);
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    if (CACHED && first < rows) fetch(first);
+    for (int row = first; row < rows; row += step) {
         const T* xr = x + (size_t)row * cols;
         T* yr = y + (size_t)row * cols;
-        float v[MAXV][8];
+        float v[CACHED ? V : 1][8];
         float s = 0.f;
-        if (cached) {
+        if (CACHED) {
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) {
-                const int c = threadIdx.x + j * blockDim.x;
+            for (int j = 0; j < V; ++j) {
+                const int c = tid + j * width;
                 if (c < nvec) {
                     Vec8<T>::unpack(nxt[j], v[j]);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) s += RMS ? v[j][i] * v[j][i] : v[j][i];
                 }
             }
-            if (row + (int)gridDim.x < rows) fetch(row + gridDim.x);
+            if (row + step < rows) fetch(row + step);
         } else {
-            for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
+            for (int c = tid; c < nvec; c += width) {
                 float t[8];
                 Vec8<T>::load(xr + c * 8, t);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) s += RMS ? t[i] * t[i] : t[i];
             }
         }
-        s = block_sum(s, red);
         float mean = 0.f, scale;
         if (RMS) {
+            s = row_sum<WARP>(s, (row / step) & 1 ? red1 : red0);
             scale = 1.0f / (sqrtf(s / cols) + eps);
         } else {
+            s = row_sum<WARP>(s, red0);
             mean = s / cols;
             float q = 0.f;
-            if (cached) {
+            if (CACHED) {
 #pragma unroll
-                for (int j = 0; j < MAXV; ++j) {
-                    const int c = threadIdx.x + j * blockDim.x;
+                for (int j = 0; j < V; ++j) {
+                    const int c = tid + j * width;
                     if (c < nvec) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
@@ -216,7 +222,7 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const T* __restrict__ x, 
                     }
                 }
             } else {
-                for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
+                for (int c = tid; c < nvec; c += width) {
                     float t[8];
                     Vec8<T>::load(xr + c * 8, t);
 #pragma unroll
@@ -226,10 +232,10 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const T* __restrict__ x, 
                     }
                 }
             }
-            q = block_sum(q, red);
+            q = row_sum<WARP>(q, red1);
             scale = rsqrtf(q / cols + eps);
         }
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
             if (stat0) stat0[row] = mean;
             stat1[row] = scale;
         }
@@ -241,14 +247,14 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const T* __restrict__ x, 
             for (int i = 0; i < 8; ++i) o[i] = (t[i] - mean) * scale * g[i] + (beta ? b[i] : 0.f);
             Vec8<T>::store(yr + c * 8, o);
         };
-        if (cached) {
+        if (CACHED) {
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) {
-                const int c = threadIdx.x + j * blockDim.x;
+            for (int j = 0; j < V; ++j) {
+                const int c = tid + j * width;
                 if (c < nvec) emit(c, v[j]);
             }
         } else {
-            for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
+            for (int c = tid; c < nvec; c += width) {
                 float t[8];
                 Vec8<T>::load(xr + c * 8, t);
                 emit(c, t);
@@ -257,88 +263,89 @@ __global__ void __launch_bounds__(256) norm_fwd_kernel(const T* __restrict__ x, 
     }
 }
 
-// Backward.  Column sums (dgamma, dbeta) are accumulated per CTA in registers (cached path) or in
-// global partial rows (generic path) and written to partial[blockIdx.x][cols]; a second kernel
-// reduces the partial rows.  partial layout: [2][nblk][cols] fp32.
-template <typename T, bool RMS>
-__global__ void __launch_bounds__(256) norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x,
-                                                       const T* __restrict__ gamma, const float* __restrict__ stat0,
-                                                       const float* __restrict__ stat1, T* dx,
-                                                       float* __restrict__ partial, int rows, int cols, float eps,
-                                                       const T* add) {
+// Backward.  Column sums (dgamma, dbeta) are accumulated in registers (V > 0) or in global partial rows (generic path)
+// and written to partial[blockIdx.x][cols]; a second kernel reduces the partial rows.  partial layout: [2][nblk][cols]
+// fp32.  The current row stays packed between its two uses (statistics, output), which halves the registers it takes.
+template <typename T, bool RMS, int V>
+__global__ void __launch_bounds__(CTA_THREADS, sizeof(T) == 2 && V < 3 ? 2 : 1)
+norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __restrict__ gamma,
+                const float* __restrict__ stat0, const float* __restrict__ stat1, T* dx, float* __restrict__ partial,
+                int rows, int cols, float eps, const T* add) {
     // add (optional, may alias dx): dx = gradient through the norm + add -- lets the caller fold the other
     // gradient contributions of the norm's input (residual path, a sibling norm) into this pass
-    __shared__ float red[66];
+    __shared__ float2 red0[32], red1[32];
+    constexpr bool CACHED = V > 0;
+    constexpr int VV = CACHED ? V : 1;
     const int nvec = cols >> 3;
-    const bool cached = nvec <= MAXV * (int)blockDim.x;
+    const int tid = threadIdx.x, width = blockDim.x, first = blockIdx.x, step = gridDim.x;
     float* pg = partial + (size_t)blockIdx.x * cols;
     float* pb = partial + ((size_t)gridDim.x + blockIdx.x) * cols;
-    float ag[MAXV][8], ab[MAXV][8];
-    if (cached) {
+    float ag[VV][8], ab[VV][8];
+    if (CACHED) {
 #pragma unroll
-        for (int j = 0; j < MAXV; ++j)
+        for (int j = 0; j < V; ++j)
 #pragma unroll
             for (int i = 0; i < 8; ++i) ag[j][i] = ab[j][i] = 0.f;
     } else {
         for (int c = threadIdx.x; c < cols; c += blockDim.x) pg[c] = pb[c] = 0.f;
+        __syncthreads();
     }
-    typename Vec8<T>::Raw nx[MAXV], ng[MAXV];      // next row, packed (see the forward kernel)
+    typename Vec8<T>::Raw nx[VV], ng[VV];           // next row, packed
     float n_mean = 0.f, n_sc = 0.f;                 // ... and its saved statistics
     auto fetch = [&](int r) {
         n_mean = RMS ? 0.f : stat0[r];
         n_sc = stat1[r];
 #pragma unroll
-        for (int j = 0; j < MAXV; ++j) {
-            const int c = threadIdx.x + j * blockDim.x;
+        for (int j = 0; j < V; ++j) {
+            const int c = tid + j * width;
             if (c < nvec) {
                 nx[j] = Vec8<T>::raw_load(x + (size_t)r * cols + c * 8);
                 ng[j] = Vec8<T>::raw_load(g + (size_t)r * cols + c * 8);
             }
         }
     };
-    if (cached && (int)blockIdx.x < rows) fetch(blockIdx.x);
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    if (CACHED && first < rows) fetch(first);
+    for (int row = first; row < rows; row += step) {
         const T* xr = x + (size_t)row * cols;
         const T* gr = g + (size_t)row * cols;
         T* dr = dx + (size_t)row * cols;
         float mean, sc;
         float s1 = 0.f, s2 = 0.f;
-        float xv[MAXV][8], gv[MAXV][8];
-        if (cached) {
+        typename Vec8<T>::Raw cx[VV], cgr[VV], ca[VV];
+        if (CACHED) {
             mean = n_mean;
             sc = n_sc;
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) {
-                const int c = threadIdx.x + j * blockDim.x;
-                if (c < nvec) {
-                    Vec8<T>::unpack(nx[j], xv[j]);
-                    Vec8<T>::unpack(ng[j], gv[j]);
-                }
+            for (int j = 0; j < V; ++j) {
+                cx[j] = nx[j];
+                cgr[j] = ng[j];
+                const int c = tid + j * width;
+                if (add && c < nvec) ca[j] = Vec8<T>::raw_load(add + (size_t)row * cols + c * 8);
             }
-            if (row + (int)gridDim.x < rows) fetch(row + gridDim.x);
+            if (row + step < rows) fetch(row + step);
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) {
-                const int c = threadIdx.x + j * blockDim.x;
+            for (int j = 0; j < V; ++j) {
+                const int c = tid + j * width;
                 if (c < nvec) {
-                    float gm[8];
+                    float gm[8], xv[8], gv[8];
                     Vec8<T>::load(gamma + c * 8, gm);
+                    Vec8<T>::unpack(cx[j], xv);
+                    Vec8<T>::unpack(cgr[j], gv);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        const float xh = RMS ? xv[j][i] : (xv[j][i] - mean) * sc;
-                        const float gg = gv[j][i] * gm[i];
+                        const float xh = RMS ? xv[i] : (xv[i] - mean) * sc;
+                        const float gg = gv[i] * gm[i];
                         s1 += gg;
                         s2 += gg * xh;
-                        ag[j][i] += gv[j][i] * (RMS ? xv[j][i] * sc : xh);
-                        ab[j][i] += gv[j][i];
-                        gv[j][i] = gg;   // keep g*gamma
-                        xv[j][i] = xh;   // keep xhat (LN) or x (RMS)
+                        ag[j][i] += gv[i] * (RMS ? xv[i] * sc : xh);
+                        ab[j][i] += gv[i];
                     }
                 }
             }
         } else {
             mean = RMS ? 0.f : stat0[row];
             sc = stat1[row];
-            for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
+            for (int c = tid; c < nvec; c += width) {
                 float xt[8], gt[8], gm[8];
                 Vec8<T>::load(xr + c * 8, xt);
                 Vec8<T>::load(gr + c * 8, gt);
@@ -354,7 +361,7 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const T* __restrict__ g, 
                 }
             }
         }
-        block_sum2(s1, s2, red);
+        block_sum2(s1, s2, (row / step) & 1 ? red1 : red0);
         // LN : dx = sc * (gg - s1/n - xhat * s2/n)
         // RMS: y = x*sc*gamma, sc = 1/(r+eps), r = sqrt(mean x^2) -> dx = gg*sc - x * s2 * sc^2 / (n * r)
         float k1, k2;
@@ -366,43 +373,43 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const T* __restrict__ g, 
             k1 = s1 / cols;
             k2 = s2 / cols;
         }
-        auto emit = [&](int c, const float (&xh)[8], const float (&gg)[8]) {
-            float o[8];
+        auto emit = [&](int c, const float (&xt)[8], const float (&gt)[8], const float (&a8)[8]) {
+            float o[8], gm[8];
+            Vec8<T>::load(gamma + c * 8, gm);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = RMS ? gg[i] * sc - xh[i] * k2 : sc * (gg[i] - k1 - xh[i] * k2);
-            if (add) {
-                float a8[8];
-                Vec8<T>::load(add + (size_t)row * cols + c * 8, a8);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] += a8[i];
+            for (int i = 0; i < 8; ++i) {
+                const float xh = RMS ? xt[i] : (xt[i] - mean) * sc, gg = gt[i] * gm[i];
+                o[i] = RMS ? gg * sc - xh * k2 : sc * (gg - k1 - xh * k2);
+                if (add) o[i] += a8[i];
             }
             Vec8<T>::store(dr + c * 8, o);
         };
-        if (cached) {
+        if (CACHED) {
 #pragma unroll
-            for (int j = 0; j < MAXV; ++j) {
-                const int c = threadIdx.x + j * blockDim.x;
-                if (c < nvec) emit(c, xv[j], gv[j]);
+            for (int j = 0; j < V; ++j) {
+                const int c = tid + j * width;
+                if (c < nvec) {
+                    float xt[8], gt[8], a8[8];
+                    Vec8<T>::unpack(cx[j], xt);
+                    Vec8<T>::unpack(cgr[j], gt);
+                    if (add) Vec8<T>::unpack(ca[j], a8);
+                    emit(c, xt, gt, a8);
+                }
             }
         } else {
-            for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
-                float xt[8], gt[8], gm[8], xh[8], gg[8];
+            for (int c = tid; c < nvec; c += width) {
+                float xt[8], gt[8], a8[8];
                 Vec8<T>::load(xr + c * 8, xt);
                 Vec8<T>::load(gr + c * 8, gt);
-                Vec8<T>::load(gamma + c * 8, gm);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    xh[i] = RMS ? xt[i] : (xt[i] - mean) * sc;
-                    gg[i] = gt[i] * gm[i];
-                }
-                emit(c, xh, gg);
+                if (add) Vec8<T>::load(add + (size_t)row * cols + c * 8, a8);
+                emit(c, xt, gt, a8);
             }
         }
     }
-    if (cached) {
+    if constexpr (CACHED) {
 #pragma unroll
-        for (int j = 0; j < MAXV; ++j) {
-            const int c = threadIdx.x + j * blockDim.x;
+        for (int j = 0; j < V; ++j) {
+            const int c = tid + j * width;
             if (c < nvec) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -414,17 +421,125 @@ __global__ void __launch_bounds__(256) norm_bwd_kernel(const T* __restrict__ g, 
     }
 }
 
-// out0[c] = sum_r partial[r][c], out1[c] = sum_r partial[nblk + r][c].  A CTA owns 32 columns; its 8 warps take
-// every 8th partial row (coalesced 128-byte reads), then the 8 row lanes are added in a fixed order -- about 190 CTAs
-// for 6144 columns instead of the 24 a thread-per-column loop gave, which was latency-bound on ~600 serial loads.
-__global__ void __launch_bounds__(256) colreduce_kernel(const float* __restrict__ partial, float* __restrict__ out0,
-                                                        float* __restrict__ out1, int nblk, int cols) {
-    __shared__ float sa[8][33], sb[8][33];
+// Backward of rows of up to 1024 columns.  A row belongs to G = 1 to 4 warps (one vector of 8 a lane, so that the whole
+// state of a thread is 64 registers), a CTA of 16 warps to 16 / G rows; two CTAs fill an SM.  The warps of a row meet at a
+// barrier of their own, the row groups of a CTA only at the end, for the column sums.
+constexpr int ROWS_THREADS = 512;
+template <typename T, bool RMS, int G>
+__global__ void __launch_bounds__(ROWS_THREADS, sizeof(T) == 2 ? 2 : 1)
+norm_bwd_rows_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __restrict__ gamma,
+                     const float* __restrict__ stat0, const float* __restrict__ stat1, T* dx, float* __restrict__ partial,
+                     int rows, int cols, float eps, const T* add) {
+    constexpr int GROUPS = ROWS_THREADS / 32 / G, WIDTH = G * 32;
+    __shared__ float2 red[2][GROUPS][G];
+    __shared__ float sums[2][GROUPS][WIDTH * 8];
+    const int group = threadIdx.x / WIDTH, tid = threadIdx.x % WIDTH;       // the warps left over (G = 3) have no rows
+    const int step = gridDim.x * GROUPS, first = group < GROUPS ? group * gridDim.x + blockIdx.x : rows;
+    const bool has = tid * 8 < cols;
+    float ag[8], ab[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ag[i] = ab[i] = 0.f;
+    typename Vec8<T>::Raw nx, ng, rgm;
+    if (has) rgm = Vec8<T>::raw_load(gamma + tid * 8);
+    float n_mean = 0.f, n_sc = 0.f;
+    auto fetch = [&](int r) {
+        n_mean = RMS ? 0.f : stat0[r];
+        n_sc = stat1[r];
+        if (has) {
+            nx = Vec8<T>::raw_load(x + (size_t)r * cols + tid * 8);
+            ng = Vec8<T>::raw_load(g + (size_t)r * cols + tid * 8);
+        }
+    };
+    if (first < rows) fetch(first);
+    for (int row = first, turn = 0; row < rows; row += step, turn ^= 1) {
+        const float mean = n_mean, sc = n_sc;
+        float xv[8], gv[8], s1 = 0.f, s2 = 0.f;
+        typename Vec8<T>::Raw ca;
+        if (has) {
+            Vec8<T>::unpack(nx, xv);
+            Vec8<T>::unpack(ng, gv);
+            if (add) ca = Vec8<T>::raw_load(add + (size_t)row * cols + tid * 8);
+        }
+        if (row + step < rows) fetch(row + step);
+        if (has) {
+            float gm[8];
+            Vec8<T>::unpack(rgm, gm);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float xh = RMS ? xv[i] : (xv[i] - mean) * sc;
+                const float gg = gv[i] * gm[i];
+                s1 += gg;
+                s2 += gg * xh;
+                ag[i] += gv[i] * (RMS ? xv[i] * sc : xh);
+                ab[i] += gv[i];
+                gv[i] = gg;
+                xv[i] = xh;
+            }
+        }
+        s1 = warp_sum(s1);
+        s2 = warp_sum(s2);
+        if constexpr (G > 1) {
+            if ((tid & 31) == 0) red[turn][group][tid >> 5] = make_float2(s1, s2);
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(WIDTH) : "memory");
+            s1 = s2 = 0.f;
+#pragma unroll
+            for (int w = 0; w < G; ++w) {
+                s1 += red[turn][group][w].x;
+                s2 += red[turn][group][w].y;
+            }
+        }
+        // (the formulas of norm_bwd_kernel)
+        float k1, k2;
+        if (RMS) {
+            const float r = 1.0f / sc - eps;
+            k1 = 0.f;
+            k2 = (r > 0.f) ? s2 * sc * sc / (cols * r) : 0.f;
+        } else {
+            k1 = s1 / cols;
+            k2 = s2 / cols;
+        }
+        if (has) {
+            float o[8], a8[8];
+            if (add) Vec8<T>::unpack(ca, a8);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                o[i] = RMS ? gv[i] * sc - xv[i] * k2 : sc * (gv[i] - k1 - xv[i] * k2);
+                if (add) o[i] += a8[i];
+            }
+            Vec8<T>::store(dx + (size_t)row * cols + tid * 8, o);
+        }
+    }
+    if (group < GROUPS) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            sums[0][group][tid * 8 + i] = ag[i];
+            sums[1][group][tid * 8 + i] = ab[i];
+        }
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < 2 * cols; c += ROWS_THREADS) {
+        const int which = c >= cols, col = which ? c - cols : c;
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < GROUPS; ++q) v += sums[which][q][col];          // a fixed order
+        partial[((size_t)which * gridDim.x + blockIdx.x) * cols + col] = v;
+    }
+}
+
+// out0[c] (+)= sum_r partial[r][c], out1[c] (+)= sum_r partial[nblk + r][c].  A CTA owns 32 columns; its 32 warps take
+// every 32nd partial row (coalesced 128-byte reads), then the 32 row lanes are added in a fixed order.  The loads of a
+// thread are serial, so what counts is how few each has: 10 of 296 rows; with 8 warps (37 rows) it took 6.1 us.
+constexpr int RED_WARPS = 32;
+__global__ void __launch_bounds__(RED_WARPS * 32)
+colreduce_kernel(const float* __restrict__ partial, float* __restrict__ out0, float* __restrict__ out1, int nblk, int cols,
+                 int acc0, int acc1) {
+    __shared__ float sa[RED_WARPS][33], sb[RED_WARPS][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int c = blockIdx.x * 32 + tx;
     float a = 0.f, b = 0.f;
     if (c < cols) {
-        for (int r = ty; r < nblk; r += 8) {
+#pragma unroll 5
+        for (int r = ty; r < nblk; r += RED_WARPS) {
             a += partial[(size_t)r * cols + c];
             b += partial[((size_t)nblk + r) * cols + c];
         }
@@ -432,22 +547,49 @@ __global__ void __launch_bounds__(256) colreduce_kernel(const float* __restrict_
     sa[ty][tx] = a;
     sb[ty][tx] = b;
     __syncthreads();
-    if (ty == 0 && c < cols) {
-        float ta = 0.f, tb = 0.f;
+    if (ty < 2 && c < cols) {
+        float t = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            ta += sa[j][tx];
-            tb += sb[j][tx];
-        }
-        out0[c] = ta;
-        if (out1) out1[c] = tb;
+        for (int j = 0; j < RED_WARPS; ++j) t += ty ? sb[j][tx] : sa[j][tx];
+        float* out = ty ? out1 : out0;
+        if (out) out[c] = (ty ? acc1 : acc0) ? out[c] + t : t;
     }
 }
 
-int pick_threads(int cols) {
-    int t = 32;
-    while (t < 256 && t * 8 < cols) t <<= 1;
-    return t;
+// Calls f with the kernel's template arguments for this row length as f(V, WARP); rows of up to 1024 columns: V vectors of a
+// warp's lanes forward, V warps backward.
+template <typename F>
+int for_row_length(int cols, F f) {
+    using std::integral_constant;
+    const int nvec = cols / 8;
+    constexpr integral_constant<bool, true> warp{};
+    constexpr integral_constant<bool, false> cta{};
+    if (cols <= ROW_COLS) {
+        if (nvec <= 32) return f(integral_constant<int, 1>{}, warp);
+        if (nvec <= 64) return f(integral_constant<int, 2>{}, warp);
+        if (nvec <= 96) return f(integral_constant<int, 3>{}, warp);
+        return f(integral_constant<int, 4>{}, warp);
+    }
+    if (nvec <= CTA_THREADS) return f(integral_constant<int, 1>{}, cta);
+    if (nvec <= 2 * CTA_THREADS) return f(integral_constant<int, 2>{}, cta);
+    if (nvec <= 3 * CTA_THREADS) return f(integral_constant<int, 3>{}, cta);
+    return f(integral_constant<int, 0>{}, cta);
+}
+
+// Threads of a CTA that holds a row in V vectors per thread.
+int cta_threads(int nvec, int v) { return v ? ((nvec + v - 1) / v + 31) / 32 * 32 : 256; }
+
+template <typename T, bool RMS>
+int launch_norm_fwd_t(const void* x, const void* gamma, const void* beta, void* y, float* s0, float* s1, int rows, int cols,
+                      float eps, cudaStream_t st) {
+    return for_row_length(cols, [&](auto v, auto warp) {
+        constexpr int V = decltype(v)::value;
+        constexpr bool WARP = decltype(warp)::value;
+        const int blocks = WARP ? (rows + ROW_WARPS - 1) / ROW_WARPS : rows, most = neox_sm_count() * 8;
+        norm_fwd_kernel<T, RMS, V, WARP><<<blocks < most ? blocks : most, WARP ? ROW_WARPS * 32 : cta_threads(cols / 8, V), 0, st>>>(
+            (const T*)x, (const T*)gamma, (const T*)beta, (T*)y, s0, s1, rows, cols, eps);
+        return 0;
+    });
 }
 
 template <bool RMS>
@@ -455,34 +597,39 @@ int launch_norm_fwd(const void* x, const void* gamma, const void* beta, void* y,
                     int cols, float eps, int dtype, cudaStream_t st) {
     if (cols % 8) return NEOX_ERR_SHAPE;
     if (rows <= 0) return 0;
-    const int threads = pick_threads(cols);
-    const int grid = rows < neox_sm_count() * 8 ? rows : neox_sm_count() * 8;
-#define LAUNCH(T)                                                                                                   \
-    norm_fwd_kernel<T, RMS><<<grid, threads, 0, st>>>((const T*)x, (const T*)gamma, (const T*)beta, (T*)y, s0, s1, \
-                                                      rows, cols, eps)
-    if (dtype == 0) LAUNCH(__nv_bfloat16);
-    else if (dtype == 1) LAUNCH(float);
-    else LAUNCH(__half);
-#undef LAUNCH
+    if (dtype == 0) launch_norm_fwd_t<__nv_bfloat16, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
+    else if (dtype == 1) launch_norm_fwd_t<float, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
+    else launch_norm_fwd_t<__half, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
+template <typename T, bool RMS>
+void launch_norm_bwd_t(const void* g, const void* x, const void* gamma, const float* s0, const float* s1, void* dx, float* ws,
+                       int rows, int cols, float eps, cudaStream_t st, const void* add, int nblk) {
+    for_row_length(cols, [&](auto v, auto warp) {
+        constexpr int V = decltype(v)::value;
+        if constexpr (decltype(warp)::value)
+            norm_bwd_rows_kernel<T, RMS, V><<<nblk, ROWS_THREADS, 0, st>>>((const T*)g, (const T*)x, (const T*)gamma, s0, s1,
+                                                                          (T*)dx, ws, rows, cols, eps, (const T*)add);
+        else
+            norm_bwd_kernel<T, RMS, V><<<nblk, cta_threads(cols / 8, V), 0, st>>>(
+                (const T*)g, (const T*)x, (const T*)gamma, s0, s1, (T*)dx, ws, rows, cols, eps, (const T*)add);
+        return 0;
+    });
+}
+
+// d0 / d1: parameter gradients, stored, or with acc0 / acc1 added to what is there (the optimizer's fp32 gradient buffer).
 template <bool RMS>
 int launch_norm_bwd(const void* g, const void* x, const void* gamma, const float* s0, const float* s1, void* dx,
                     float* d0, float* d1, float* ws, int rows, int cols, float eps, int dtype, cudaStream_t st,
-                    const void* add = nullptr) {
+                    const void* add = nullptr, int acc0 = 0, int acc1 = 0) {
     if (cols % 8) return NEOX_ERR_SHAPE;
     if (rows <= 0) return 0;
-    const int threads = pick_threads(cols);
     const int nblk = neox_norm_bwd_blocks(rows);
-#define LAUNCH(T)                                                                                                    \
-    norm_bwd_kernel<T, RMS><<<nblk, threads, 0, st>>>((const T*)g, (const T*)x, (const T*)gamma, s0, s1, (T*)dx, ws, \
-                                                      rows, cols, eps, (const T*)add)
-    if (dtype == 0) LAUNCH(__nv_bfloat16);
-    else if (dtype == 1) LAUNCH(float);
-    else LAUNCH(__half);
-#undef LAUNCH
-    colreduce_kernel<<<(cols + 31) / 32, 256, 0, st>>>(ws, d0, d1, nblk, cols);
+    if (dtype == 0) launch_norm_bwd_t<__nv_bfloat16, RMS>(g, x, gamma, s0, s1, dx, ws, rows, cols, eps, st, add, nblk);
+    else if (dtype == 1) launch_norm_bwd_t<float, RMS>(g, x, gamma, s0, s1, dx, ws, rows, cols, eps, st, add, nblk);
+    else launch_norm_bwd_t<__half, RMS>(g, x, gamma, s0, s1, dx, ws, rows, cols, eps, st, add, nblk);
+    colreduce_kernel<<<(cols + 31) / 32, RED_WARPS * 32, 0, st>>>(ws, d0, d1, nblk, cols, acc0, acc1);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
@@ -762,18 +909,19 @@ int neox_layernorm_bwd(const void* g, const void* x, const void* gamma, const fl
     return launch_norm_bwd<false>(g, x, gamma, mean, rstd, dx, dgamma, dbeta, ws, rows, cols, 0.f, dtype,
                                   (cudaStream_t)stream);
 }
-// dx = (gradient through the norm) + add; add has the shape of dx and may be dx itself.
+// dx = (gradient through the norm) + add; add has the shape of dx and may be dx itself, or NULL.  dgamma / dbeta (may be
+// NULL) are stored, or added to with acc_gamma / acc_beta.
 int neox_layernorm_bwd_add(const void* g, const void* x, const void* gamma, const float* mean, const float* rstd,
                            void* dx, float* dgamma, float* dbeta, float* ws, int rows, int cols, int dtype,
-                           const void* add, void* stream) {
+                           const void* add, int acc_gamma, int acc_beta, void* stream) {
     return launch_norm_bwd<false>(g, x, gamma, mean, rstd, dx, dgamma, dbeta, ws, rows, cols, 0.f, dtype,
-                                  (cudaStream_t)stream, add);
+                                  (cudaStream_t)stream, add, acc_gamma, acc_beta);
 }
 int neox_rmsnorm_bwd_add(const void* g, const void* x, const void* scale, const float* rinv, void* dx, float* dscale,
                          float* dbias, float* ws, int rows, int cols, float eps, int dtype, const void* add,
-                         void* stream) {
+                         int acc_scale, int acc_bias, void* stream) {
     return launch_norm_bwd<true>(g, x, scale, nullptr, rinv, dx, dscale, dbias, ws, rows, cols, eps, dtype,
-                                 (cudaStream_t)stream, add);
+                                 (cudaStream_t)stream, add, acc_scale, acc_bias);
 }
 int neox_rmsnorm_fwd(const void* x, const void* scale, const void* bias, void* y, float* rinv, int rows, int cols,
                      float eps, int dtype, void* stream) {

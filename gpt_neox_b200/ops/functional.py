@@ -47,22 +47,49 @@ def workspace(nbytes: int, device, tag="ws") -> torch.Tensor:
     return buf
 
 
-def _param_grad(param, g32):
-    """Hand an fp32 parameter gradient to the optimizer: added to ``param.main_grad`` (the flat fp32 gradient buffer)
-    when it exists -- no round trip through the 16-bit ``.grad`` and its accumulate hook -- else returned in the
-    parameter's type."""
+def _norm_grad_target(param, cols, device):
+    """Where a norm's backward kernel puts an fp32 parameter gradient: ``(tensor, accumulate)`` -- ``param.main_grad`` (the
+    optimizer's flat fp32 gradient buffer) to add to when it exists, else a new tensor."""
     if param is None:
-        return None
+        return None, 0
     from .linear import main_grad_of
     mg = main_grad_of(param)
-    if mg is not None and mg.dtype == torch.float32 and mg.shape == g32.shape:
-        mg.add_(g32)
-        param.grad_in_main = True
-        ready = getattr(param, "_grad_ready", None)
-        if ready is not None:
-            ready()
+    if mg is not None and mg.dtype == torch.float32 and mg.shape == (cols,) and mg.is_contiguous():
+        return mg, 1
+    return torch.empty(cols, dtype=torch.float32, device=device), 0
+
+
+def _norm_grad(param, target, accumulated, wanted):
+    """What autograd gets for it: nothing once it is in ``main_grad`` (no round trip through the 16-bit ``.grad`` and its
+    accumulate hook; the parameter is reported ready), else the gradient in the parameter's type."""
+    if not wanted:
         return None
-    return g32.to(param.dtype)
+    if not accumulated:
+        return target.to(param.dtype)
+    param.grad_in_main = True
+    ready = getattr(param, "_grad_ready", None)
+    if ready is not None:
+        ready()
+    return None
+
+
+def _norm_backward(kind, g2, x2, w, b, mean, sc, dx, add, eps, want_w, want_b):
+    """One norm-backward launch (``dx = gradient + add``) plus the reduction of its parameter gradients; returns these."""
+    rows, cols = x2.shape
+    L = native.lib()
+    ws = workspace(2 * int(L.neox_norm_bwd_blocks(rows)) * cols * 4, x2.device, "ln_bwd")
+    d0, acc0 = _norm_grad_target(w if want_w else None, cols, x2.device)
+    d1, acc1 = _norm_grad_target(b if want_b else None, cols, x2.device)
+    if kind == "ln":
+        rc = L.neox_layernorm_bwd_add(native.ptr(g2), native.ptr(x2), native.ptr(w), native.ptr(mean), native.ptr(sc),
+                                      native.ptr(dx), native.ptr(d0), native.ptr(d1), native.ptr(ws), rows, cols,
+                                      _DT[x2.dtype], native.ptr(add), acc0, acc1, _s())
+    else:
+        rc = L.neox_rmsnorm_bwd_add(native.ptr(g2), native.ptr(x2), native.ptr(w), native.ptr(sc), native.ptr(dx),
+                                    native.ptr(d0), native.ptr(d1), native.ptr(ws), rows, cols, ctypes.c_float(eps),
+                                    _DT[x2.dtype], native.ptr(add), acc0, acc1, _s())
+    native.check(rc, "norm backward")
+    return _norm_grad(w, d0, acc0, want_w), _norm_grad(b, d1, acc1, want_b)
 
 
 # ------------------------------------------------------------------------------------ LayerNorm
@@ -107,16 +134,9 @@ class _LayerNormFn(torch.autograd.Function):
         if not g2.is_contiguous():
             g2 = g2.contiguous()
         dx = torch.empty_like(x2)
-        nblk = int(native.lib().neox_norm_bwd_blocks(rows))
-        ws = workspace(2 * nblk * cols * 4, x2.device, "ln_bwd")
-        dgamma = torch.empty(cols, dtype=torch.float32, device=x2.device)
-        dbeta = torch.empty(cols, dtype=torch.float32, device=x2.device)
-        rc = native.lib().neox_layernorm_bwd(native.ptr(g2), native.ptr(x2), native.ptr(weight), native.ptr(mean),
-                                             native.ptr(rstd), native.ptr(dx), native.ptr(dgamma), native.ptr(dbeta),
-                                             native.ptr(ws), rows, cols, _DT[x2.dtype], _s())
-        native.check(rc, "neox_layernorm_bwd")
-        return (dx.reshape(ctx.shape), _param_grad(weight, dgamma) if ctx.needs_input_grad[1] else None,
-                _param_grad(ctx.bias_ref, dbeta) if ctx.has_bias and ctx.needs_input_grad[2] else None, None)
+        gw, gb = _norm_backward("ln", g2, x2, weight, ctx.bias_ref, mean, rstd, dx, None, 0.0, ctx.needs_input_grad[1],
+                                ctx.has_bias and ctx.needs_input_grad[2])
+        return dx.reshape(ctx.shape), gw, gb, None
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
@@ -165,16 +185,9 @@ class _RMSNormFn(torch.autograd.Function):
         if not g2.is_contiguous():
             g2 = g2.contiguous()
         dx = torch.empty_like(x2)
-        nblk = int(native.lib().neox_norm_bwd_blocks(rows))
-        ws = workspace(2 * nblk * cols * 4, x2.device, "ln_bwd")
-        dscale = torch.empty(cols, dtype=torch.float32, device=x2.device)
-        dbias = torch.empty(cols, dtype=torch.float32, device=x2.device)
-        rc = native.lib().neox_rmsnorm_bwd(native.ptr(g2), native.ptr(x2), native.ptr(scale), native.ptr(rinv),
-                                           native.ptr(dx), native.ptr(dscale), native.ptr(dbias), native.ptr(ws),
-                                           rows, cols, ctypes.c_float(ctx.eps), _DT[x2.dtype], _s())
-        native.check(rc, "neox_rmsnorm_bwd")
-        return (dx.reshape(ctx.shape), _param_grad(scale, dscale) if ctx.needs_input_grad[1] else None,
-                _param_grad(ctx.bias_ref, dbias) if ctx.has_bias and ctx.needs_input_grad[2] else None, None)
+        gs, gb = _norm_backward("rms", g2, x2, scale, ctx.bias_ref, None, rinv, dx, None, ctx.eps, ctx.needs_input_grad[1],
+                                ctx.has_bias and ctx.needs_input_grad[2])
+        return dx.reshape(ctx.shape), gs, gb, None
 
 
 def rms_norm(x, scale, bias=None, eps=1e-8):
@@ -436,7 +449,6 @@ class _NormFanOutFn(torch.autograd.Function):
     def backward(ctx, *grads):
         x2, *stats = ctx.saved_tensors
         rows, cols = x2.shape
-        L = native.lib()
         acc = grads[-1]                                   # gradient arriving through the residual connection
         if acc is not None:
             acc = acc.reshape(rows, cols)
@@ -444,7 +456,6 @@ class _NormFanOutFn(torch.autograd.Function):
                 acc = acc.contiguous()
         dx = None
         pgrads = []
-        nblk = int(L.neox_norm_bwd_blocks(rows))
         for i, (kind, eps) in enumerate(ctx.specs):
             w, b = ctx.params[2 * i], ctx.params[2 * i + 1]
             g = grads[i]
@@ -456,22 +467,9 @@ class _NormFanOutFn(torch.autograd.Function):
                 g2 = g2.contiguous()
             if dx is None:
                 dx = torch.empty_like(x2)
-            ws = workspace(2 * nblk * cols * 4, x2.device, "ln_bwd")
-            d0 = torch.empty(cols, dtype=torch.float32, device=x2.device)
-            d1 = torch.empty(cols, dtype=torch.float32, device=x2.device)
-            if kind == "ln":
-                rc = L.neox_layernorm_bwd_add(native.ptr(g2), native.ptr(x2), native.ptr(w), native.ptr(stats[2 * i]),
-                                              native.ptr(stats[2 * i + 1]), native.ptr(dx), native.ptr(d0),
-                                              native.ptr(d1), native.ptr(ws), rows, cols, _DT[x2.dtype],
-                                              native.ptr(acc), _s())
-            else:
-                rc = L.neox_rmsnorm_bwd_add(native.ptr(g2), native.ptr(x2), native.ptr(w), native.ptr(stats[2 * i + 1]),
-                                            native.ptr(dx), native.ptr(d0), native.ptr(d1), native.ptr(ws), rows, cols,
-                                            ctypes.c_float(eps), _DT[x2.dtype], native.ptr(acc), _s())
-            native.check(rc, "norm backward")
+            pgrads += _norm_backward(kind, g2, x2, w, b, stats[2 * i], stats[2 * i + 1], dx, acc, eps,
+                                     ctx.needs_input_grad[2 + 2 * i], b is not None and ctx.needs_input_grad[3 + 2 * i])
             acc = dx
-            pgrads.append(_param_grad(w, d0) if ctx.needs_input_grad[2 + 2 * i] else None)
-            pgrads.append(_param_grad(b, d1) if b is not None and ctx.needs_input_grad[3 + 2 * i] else None)
         gx = acc.reshape(ctx.shape) if acc is not None else None
         return (gx, None, *pgrads)
 

@@ -1114,3 +1114,37 @@ def test_decode_attention_matches_rotary_append_and_attention(n, b, hq, hkv, d, 
         assert torch.equal(c[1, n], v[0])
         keep = torch.arange(cap, device=DEV) != n
         assert torch.equal(c[:, keep], cache[:, keep])
+
+
+@pytest.mark.parametrize("kind", ["ln", "rms"])
+@pytest.mark.parametrize("rows,cols,dtype", [
+    (1, 8, torch.bfloat16), (700, 256, torch.float16), (5, 264, torch.bfloat16), (3001, 520, torch.bfloat16),
+    (900, 776, torch.float32), (1300, 1024, torch.float16), (700, 1032, torch.bfloat16), (9, 3080, torch.bfloat16),
+    (650, 6152, torch.float16), (3, 9224, torch.bfloat16)])
+def test_norm_row_splits_match_fp64(kind, rows, cols, dtype):
+    """Every split of a row (one to four warps, one to three vectors of a CTA's threads, re-read rows), part-filled warps, row
+    counts that leave CTAs or row groups without a row; addend aliasing the result, parameter gradients stored and
+    accumulated.  Row results round once (half an ulp) after fp32 sums; column sums are fp32 over ``rows`` terms."""
+    torch.manual_seed(rows + cols)
+    x, g, res = (torch.randn(rows, cols, device=DEV).to(dtype) for _ in range(3))
+    w, b = (1 + 0.1 * torch.randn(cols, device=DEV)).to(dtype), (0.1 * torch.randn(cols, device=DEV)).to(dtype)
+    xr, wr, br = (t.double().requires_grad_() for t in (x, w, b))
+    if kind == "ln":
+        yr, y = torch.nn.functional.layer_norm(xr, (cols,), wr, br, 1e-5), OF.layer_norm(x, w, b, 1e-5)
+        mean, sc = xr.mean(-1), (xr.var(-1, unbiased=False) + 1e-5).rsqrt()
+    else:
+        rms = xr.pow(2).mean(-1, keepdim=True).sqrt()
+        yr, y = xr / (rms + 1e-5) * wr + br, OF.rms_norm(x, w, b, 1e-5)
+        mean, sc = None, 1 / (rms[:, 0] + 1e-5)
+    yr.backward(g.double())
+    ulp = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -18}[dtype]
+    _close(y, yr, ulp, rtol=ulp)
+    w.main_grad = torch.full((cols,), 2.0, device=DEV)
+    dx = res.clone()
+    mean, sc = (None if t is None else t.detach().float().contiguous() for t in (mean, sc))
+    gw, gb = OF._norm_backward(kind, g, x, w, b, mean, sc, dx, dx, 1e-5, True, True)
+    _close(dx, xr.grad + res.double(), ulp, rtol=ulp)
+    assert gw is None and w.grad_in_main
+    sums = 1e-5 * math.sqrt(rows) + 1e-5
+    _close(w.main_grad - 2.0, wr.grad, sums, rtol=1e-5)
+    _close(gb, br.grad, sums, rtol=1e-5 + (0 if dtype == torch.float32 else ulp))
