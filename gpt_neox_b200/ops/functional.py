@@ -105,21 +105,26 @@ def layer_norm_ref(x, weight, bias, eps):
     return y.to(x.dtype)
 
 
+def _layer_norm_values(x, weight, bias, eps):
+    """``(x as rows, result as rows, mean, 1 / std)``."""
+    cols = x.shape[-1]
+    x2 = x.reshape(-1, cols)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    rows = x2.shape[0]
+    y = torch.empty_like(x2)
+    mean, rstd = torch.empty(2, rows, dtype=torch.float32, device=x.device).unbind(0)
+    rc = native.lib().neox_layernorm_fwd(native.ptr(x2), native.ptr(weight), native.ptr(bias), native.ptr(y),
+                                         native.ptr(mean), native.ptr(rstd), rows, cols, ctypes.c_float(eps),
+                                         _DT[x.dtype], _s())
+    native.check(rc, "neox_layernorm_fwd")
+    return x2, y, mean, rstd
+
+
 class _LayerNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, eps):
-        cols = x.shape[-1]
-        x2 = x.reshape(-1, cols)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        rows = x2.shape[0]
-        y = torch.empty_like(x2)
-        mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rc = native.lib().neox_layernorm_fwd(native.ptr(x2), native.ptr(weight), native.ptr(bias), native.ptr(y),
-                                             native.ptr(mean), native.ptr(rstd), rows, cols, ctypes.c_float(eps),
-                                             _DT[x.dtype], _s())
-        native.check(rc, "neox_layernorm_fwd")
+        x2, y, mean, rstd = _layer_norm_values(x, weight, bias, eps)
         ctx.save_for_backward(x2, weight, mean, rstd)
         ctx.has_bias = bias is not None
         ctx.bias_ref = bias
@@ -141,6 +146,8 @@ class _LayerNormFn(torch.autograd.Function):
 
 def layer_norm(x, weight, bias, eps=1e-5):
     if _k(x) and weight is not None and weight.dtype == x.dtype and x.shape[-1] % 8 == 0:
+        if native.plain_call(x, weight, bias):
+            return _layer_norm_values(x, weight, bias, eps)[1].reshape(x.shape)
         return _LayerNormFn.apply(x, weight, bias, eps)
     return F.layer_norm(x, (x.shape[-1],), weight, bias, eps)
 
@@ -157,19 +164,25 @@ def rms_norm_ref(x, scale, bias, eps):
     return y.to(x.dtype)
 
 
+def _rms_norm_values(x, scale, bias, eps):
+    """``(x as rows, result as rows, 1 / (rms + eps))``."""
+    cols = x.shape[-1]
+    x2 = x.reshape(-1, cols)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    rows = x2.shape[0]
+    y = torch.empty_like(x2)
+    rinv = torch.empty(rows, dtype=torch.float32, device=x.device)
+    rc = native.lib().neox_rmsnorm_fwd(native.ptr(x2), native.ptr(scale), native.ptr(bias), native.ptr(y),
+                                       native.ptr(rinv), rows, cols, ctypes.c_float(eps), _DT[x.dtype], _s())
+    native.check(rc, "neox_rmsnorm_fwd")
+    return x2, y, rinv
+
+
 class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, scale, bias, eps):
-        cols = x.shape[-1]
-        x2 = x.reshape(-1, cols)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        rows = x2.shape[0]
-        y = torch.empty_like(x2)
-        rinv = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rc = native.lib().neox_rmsnorm_fwd(native.ptr(x2), native.ptr(scale), native.ptr(bias), native.ptr(y),
-                                           native.ptr(rinv), rows, cols, ctypes.c_float(eps), _DT[x.dtype], _s())
-        native.check(rc, "neox_rmsnorm_fwd")
+        x2, y, rinv = _rms_norm_values(x, scale, bias, eps)
         ctx.save_for_backward(x2, scale, rinv)
         ctx.has_bias = bias is not None
         ctx.bias_ref = bias
@@ -192,6 +205,8 @@ class _RMSNormFn(torch.autograd.Function):
 
 def rms_norm(x, scale, bias=None, eps=1e-8):
     if _k(x) and scale.dtype == x.dtype and x.shape[-1] % 8 == 0:
+        if native.plain_call(x, scale, bias):
+            return _rms_norm_values(x, scale, bias, eps)[1].reshape(x.shape)
         return _RMSNormFn.apply(x, scale, bias, eps)
     return rms_norm_ref(x, scale, bias, eps)
 

@@ -144,30 +144,18 @@ def gemm(a, b, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, bias=
     if act == ACT_DGELU:
         assert aux is not None and aux.shape == (M, N) and aux.dtype == dt and aux.stride(1) == 1
     L = native.lib()
-    h16 = int(dt == torch.float16)
+    h16 = 1 if dt == torch.float16 else 0
+    head = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0))
+    epilogue = (1 if out.dtype == torch.float32 else 0, None if bias is None else bias.data_ptr(),
+                *((None, 0, 0) if add is None else (add.data_ptr(), add.stride(0), 1 if add.dtype == torch.float32 else 0)),
+                *((None, 0) if pre is None else (pre.data_ptr(), pre.stride(0))),
+                *((None, 0) if aux is None else (aux.data_ptr(), aux.stride(0))), act, alpha)
     if use_skinny_kernel(M, N, K, a_mn, b_mn):
-        rc = L.neox_gemm_skinny_16(
-            native.ptr(a), native.ptr(b), native.ptr(out), M, N, K,
-            ctypes.c_longlong(a.stride(0)), ctypes.c_longlong(b.stride(0)), ctypes.c_longlong(out.stride(0)),
-            int(out.dtype == torch.float32),
-            native.ptr(bias), native.ptr(add), ctypes.c_longlong(add.stride(0) if add is not None else 0),
-            int(add is not None and add.dtype == torch.float32),
-            native.ptr(pre), ctypes.c_longlong(pre.stride(0) if pre is not None else 0),
-            native.ptr(aux), ctypes.c_longlong(aux.stride(0) if aux is not None else 0),
-            int(act), ctypes.c_float(alpha), h16, ctypes.c_void_p(native.stream_ptr()))
-        native.check(rc, "neox_gemm_skinny_16")
-        return (out, pre) if want_preact else out
-    pair = use_pair_kernel(M, N, K)
-    tail = (h16, ctypes.c_void_p(native.stream_ptr())) if pair else (None, h16, ctypes.c_void_p(native.stream_ptr()))
-    fn = L.neox_gemm_16_2cta if pair else L.neox_gemm_16
-    rc = fn(
-        native.ptr(a), native.ptr(b), native.ptr(out), M, N, K,
-        ctypes.c_longlong(a.stride(0)), ctypes.c_longlong(b.stride(0)), ctypes.c_longlong(out.stride(0)),
-        int(a_mn), int(b_mn), int(out.dtype == torch.float32),
-        native.ptr(bias), native.ptr(add), ctypes.c_longlong(add.stride(0) if add is not None else 0),
-        int(add is not None and add.dtype == torch.float32),
-        native.ptr(pre), ctypes.c_longlong(pre.stride(0) if pre is not None else 0),
-        native.ptr(aux), ctypes.c_longlong(aux.stride(0) if aux is not None else 0),
-        int(act), ctypes.c_float(alpha), *tail)
-    native.check(rc, "neox_gemm_16")
+        rc = L.neox_gemm_skinny_16(*head, *epilogue, h16, native.stream_ptr())
+    elif use_pair_kernel(M, N, K):
+        rc = L.neox_gemm_16_2cta(*head, int(a_mn), int(b_mn), *epilogue, h16, native.stream_ptr())
+    else:
+        rc = L.neox_gemm_16(*head, int(a_mn), int(b_mn), *epilogue, None, h16, native.stream_ptr())
+    if rc:
+        native.check(rc, "neox_gemm_16")
     return (out, pre) if want_preact else out

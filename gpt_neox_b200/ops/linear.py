@@ -84,6 +84,31 @@ def kernel_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     return ok
 
 
+def _linear_values(x, weight, bias, residual, act, need_pre, split_pre):
+    """``(x as rows, act(x W^T + bias) + residual as rows, pre-activation or None, native kernel used)``."""
+    N, K = weight.shape
+    x2 = x.reshape(-1, K)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    res2 = residual.reshape(-1, N) if residual is not None else None
+    use_k = kernel_ok(x2, weight) and (bias is None or bias.dtype == x2.dtype)
+    pre = None
+    if _DEAD[0] and act is None and not split_pre:
+        out = torch.empty(x2.shape[0], N, dtype=x2.dtype, device=x2.device)
+    elif use_k:
+        r = G.gemm(x2, weight, bias=bias, add=res2, act=G.ACT_GELU if act == "gelu" else G.ACT_NONE, want_preact=need_pre)
+        out, pre = r if need_pre else (r, None)
+    else:
+        flop_count.gemm(x2.shape[0], N, x2.shape[1])
+        out = F.linear(x2, weight, bias)
+        if act == "gelu":
+            pre = out if need_pre else None
+            out = F.gelu(out, approximate="tanh")
+        if res2 is not None:
+            out = out + res2
+    return x2, out, pre, use_k
+
+
 class _LinearFn(torch.autograd.Function):
     """``split_pre``: also return the pre-activation (non-differentiable) and expect the incoming gradient to be
     w.r.t. the PRE-activation already.  ``dgelu_aux``: the pre-activation of the layer that produced ``x``; the data
@@ -99,28 +124,8 @@ class _LinearFn(torch.autograd.Function):
         # of its size (a full pass over [tokens, 4h]) for it
         ctx.set_materialize_grads(False)
         N, K = weight.shape
-        x2 = x.reshape(-1, K)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        res2 = residual.reshape(-1, N) if residual is not None else None
         need_pre = act == "gelu" and any(ctx.needs_input_grad[:3])
-        use_k = kernel_ok(x2, weight) and (bias is None or bias.dtype == x2.dtype)
-        ctx.use_k = use_k
-        pre = None
-        if _DEAD[0] and act is None and not split_pre:
-            out = torch.empty(x2.shape[0], N, dtype=x2.dtype, device=x2.device)
-        elif use_k:
-            r = G.gemm(x2, weight, bias=bias, add=res2, act=G.ACT_GELU if act == "gelu" else G.ACT_NONE,
-                       want_preact=need_pre)
-            out, pre = r if need_pre else (r, None)
-        else:
-            flop_count.gemm(x2.shape[0], N, x2.shape[1])
-            out = F.linear(x2, weight, bias)
-            if act == "gelu":
-                pre = out if need_pre else None
-                out = F.gelu(out, approximate="tanh")
-            if res2 is not None:
-                out = out + res2
+        x2, out, pre, ctx.use_k = _linear_values(x, weight, bias, residual, act, need_pre, split_pre)
         ctx.has_bias = bias is not None
         ctx.bias_ref = bias
         ctx.has_res = residual is not None
@@ -187,4 +192,7 @@ class _LinearFn(torch.autograd.Function):
 def linear(x, weight, bias=None, residual=None, act=None, dgelu_aux=None, split_pre=False):
     """``act(x @ weight.T + bias) + residual`` with the epilogue fused into the GEMM (see ``_LinearFn`` for the
     two GeLU-backward options)."""
+    if native.plain_call(x, weight, bias, residual):
+        out = _linear_values(x, weight, bias, residual, act, False, split_pre)[1].reshape(*x.shape[:-1], weight.shape[0])
+        return (out, None) if split_pre else out
     return _LinearFn.apply(x, weight, bias, residual, act, dgelu_aux, split_pre)

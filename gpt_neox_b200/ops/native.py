@@ -11,6 +11,7 @@ import os
 from pathlib import Path
 
 import torch
+from torch.autograd import forward_ad
 
 _LIBDIR = Path(__file__).resolve().parent / "_lib"
 _cuda_lib = None
@@ -35,6 +36,16 @@ def _load(name: str, builder: str):
     return ctypes.CDLL(str(path))
 
 
+# The entry points of every linear layer, with their argument types declared: plain integers (addresses, strides) are then
+# converted by ctypes itself, which is cheaper than wrapping each of some twenty in an object.
+_GEMM_HEAD = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_ll, c_ll, c_ll]
+_GEMM_EPILOGUE = [c_int, c_void_p, c_void_p, c_ll, c_int, c_void_p, c_ll, c_void_p, c_ll, c_int, c_float]
+_ARGTYPES = {
+    "neox_gemm_skinny_16": [*_GEMM_HEAD, *_GEMM_EPILOGUE, c_int, c_void_p],
+    "neox_gemm_16": [*_GEMM_HEAD, c_int, c_int, *_GEMM_EPILOGUE, c_void_p, c_int, c_void_p],
+    "neox_gemm_16_2cta": [*_GEMM_HEAD, c_int, c_int, *_GEMM_EPILOGUE, c_int, c_void_p],
+}
+
 launch_count = 0   # number of kernel-launching library calls made by this process (see bench.py)
 
 
@@ -51,6 +62,8 @@ class _CountingLib:
         fn = self._cache.get(name)
         if fn is None:
             raw = getattr(self._cdll, name)
+            if name in _ARGTYPES:
+                raw.argtypes = _ARGTYPES[name]
             if name in self._NOT_LAUNCHES:
                 fn = raw
             else:
@@ -81,13 +94,35 @@ def host_lib():
     return _host_lib
 
 
+_cuda_seen = False
+
+
 def available() -> bool:
-    """True when kernels can run: a CUDA device is visible (the library itself must then load)."""
-    return torch.cuda.is_available()
+    """True when kernels can run: a CUDA device is visible (the library itself must then load).  Asked on every call of every
+    operator, and the driver query behind it takes 4 us: once a device has been seen it is not asked again."""
+    global _cuda_seen
+    if not _cuda_seen:
+        _cuda_seen = torch.cuda.is_available()
+    return _cuda_seen
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device, without the Stream object that ``torch.cuda.current_stream()``
+    builds around it (15 us)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def plain_call(*tensors) -> bool:
+    """May an operator compute its values directly instead of going through ``torch.autograd.Function`` (20 us of a decoding
+    step's launch)?  Only where that makes no difference: nothing records gradients, no functorch transform, forward-mode
+    level or tracer is active, and the arguments are plain tensors."""
+    if torch.is_grad_enabled() or torch._C._functorch.peek_interpreter_stack() is not None \
+            or forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None:
+        return False
+    for t in tensors:
+        if t is not None and type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter:
+            return False
+    return True
 
 
 def ptr(t):

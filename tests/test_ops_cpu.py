@@ -127,3 +127,39 @@ def test_cpu_adam_host_kernel_matches_torch(adamw):
     assert p.data_ptr() == storage and "host_param" not in ours.state[p]
     torch.testing.assert_close(p.detach(), q.detach(), atol=2e-6, rtol=1e-5)
     assert torch.equal(p.model_out, p.detach().bfloat16())
+
+
+def test_plain_calls_leave_transforms_to_autograd():
+    """Operators pass autograd.Function by only where nothing can tell the difference: gradients off, no functorch transform,
+    no forward-mode level, plain tensors."""
+    from torch.autograd import forward_ad
+    from gpt_neox_b200.ops import native
+
+    class Sub(torch.Tensor):
+        pass
+    x = torch.randn(3)
+    assert not native.plain_call(x)
+    seen = []
+    with torch.no_grad():
+        assert native.plain_call(x, None, torch.nn.Parameter(x))
+        assert not native.plain_call(x, x.as_subclass(Sub))
+        torch.func.vmap(lambda t: seen.append(native.plain_call(x)) or t)(x)
+        with forward_ad.dual_level():
+            seen.append(native.plain_call(x))
+        torch.jit.trace(lambda t: (seen.append(native.plain_call(x)), t * 2)[1], (x,), check_trace=False)
+    assert seen == [False] * len(seen) and len(seen) >= 3
+
+
+def test_linear_without_gradients_equals_the_recorded_one():
+    """The direct path of ``linear`` (no autograd node) gives the values of the recorded one, for every epilogue."""
+    from gpt_neox_b200.ops.linear import linear
+    torch.manual_seed(0)
+    x, w, b, r = torch.randn(2, 5, 16), torch.randn(24, 16, requires_grad=True), torch.randn(24), torch.randn(2, 5, 24)
+    for kw in ({}, {"bias": b}, {"bias": b, "act": "gelu"}, {"bias": b, "residual": r}, {"bias": b, "act": "gelu", "split_pre": True}):
+        with_graph = linear(x, w, **kw)
+        with torch.no_grad():
+            without = linear(x, w, **kw)
+        if kw.get("split_pre"):
+            assert without[1] is None
+            with_graph, without = with_graph[0], without[0]
+        assert with_graph.requires_grad and not without.requires_grad and torch.equal(with_graph, without)
