@@ -1148,3 +1148,69 @@ def test_norm_row_splits_match_fp64(kind, rows, cols, dtype):
     sums = 1e-5 * math.sqrt(rows) + 1e-5
     _close(w.main_grad - 2.0, wr.grad, sums, rtol=1e-5)
     _close(gb, br.grad, sums, rtol=1e-5 + (0 if dtype == torch.float32 else ulp))
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 256, 8192), (136, 40, 4104), (768, 768, 1000), (72, 1032, 3000), (2048, 2048, 1024)])
+def test_accumulating_gemm_splits_the_contraction(M, N, K):
+    """``acc += a^T b`` where few output tiles make the kernel split K (up to 8 parts, uneven, ragged edges of the output in
+    element-wise additions) and where it does not.  fp32 accumulation: error below sqrt(K) * 2^-22 of the terms' size."""
+    from gpt_neox_b200.ops import gemm as G
+    torch.manual_seed(K)
+    a, b = torch.randn(K, M, device=DEV).to(torch.bfloat16), torch.randn(K, N, device=DEV).to(torch.bfloat16)
+    acc = torch.randn(M, N, device=DEV)
+    want = acc.double() + a.double().t() @ b.double()
+    G.gemm(a, b, a_mn=True, b_mn=True, out=acc, add=acc)
+    _close(acc, want, 1e-5 * math.sqrt(K), rtol=1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("s,b,hq,hk,d,rot", [(7, 3, 5, 5, 64, 64), (33, 1, 3, 1, 96, 24), (5, 2, 4, 4, 128, 32), (9, 1, 2, 2, 64, 20),
+                                             (4, 1, 1, 1, 96, 6)])
+def test_rope_in_place_every_access_width(s, b, hq, hk, d, rot, dtype):
+    """In-place rotation of q and k inside a packed projection: vectors of 8 and 4 and single elements, head counts that leave
+    a thread's group of four part full, and the inverse.  One rounding, half an ulp, after two products in fp32 that may cancel:
+    2^-24 of each product's size, with and without a fused multiply-add."""
+    import ctypes
+    torch.manual_seed(rot)
+    packed = torch.randn(s, b, hq + 2 * hk, d, device=DEV).to(dtype)
+    before = packed.clone()
+    q, k = packed[:, :, :hq], packed[:, :, hq:hq + hk]
+    cos, sin = torch.randn(s, rot, device=DEV), torch.randn(s, rot, device=DEV)
+    ll = ctypes.c_longlong
+    ulp = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -20}[dtype]
+    for inverse in (0, 1):
+        want = OF.rope_ref(packed[:, :, :hq + hk], cos.view(s, 1, 1, rot), (-sin if inverse else sin).view(s, 1, 1, rot))
+        native.check(native.lib().neox_rope_qk_inplace(
+            native.ptr(q), native.ptr(k), native.ptr(cos), native.ptr(sin), s, b, hq, hk, rot, ll(q.stride(0)),
+            ll(q.stride(1)), ll(q.stride(2)), ll(k.stride(0)), ll(k.stride(1)), ll(k.stride(2)), inverse, OF._DT[dtype],
+            OF._s()), "rope")
+        products = 2.0 ** -22 * before.float().abs().max().item() * max(cos.abs().max().item(), sin.abs().max().item()) ** 2
+        _close(packed[:, :, :hq + hk], want, ulp / 8 + products, rtol=ulp)
+        assert torch.equal(packed[:, :, hq + hk:], before[:, :, hq + hk:])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n,offset", [(1, 0), (4, 0), (1027, 0), (1027, 4), (1027, 1), (300000, 0), (300000, 2)])
+def test_adam_shards_of_any_alignment(n, offset, dtype):
+    """A shard that starts anywhere in a flat buffer: four elements at a time where all tensors allow it, one otherwise, the
+    remainder, and nothing outside the shard.  The update in fp64, fp32 rounding of a few operations."""
+    import ctypes
+    torch.manual_seed(n)
+    full = n + offset + 8
+    p, m, g = (torch.randn(full, device=DEV) for _ in range(3))
+    v, out = torch.rand(full, device=DEV), torch.zeros(full, device=DEV, dtype=dtype)
+    keep = [t.clone() for t in (p, m, v, out)]
+    sl = slice(offset, offset + n)
+    f = ctypes.c_float
+    native.check(native.lib().neox_adam_step(
+        native.ptr(p[sl]), native.ptr(m[sl]), native.ptr(v[sl]), native.ptr(g[sl]), native.ptr(out[sl]), OF._DT[dtype],
+        ctypes.c_longlong(n), f(1e-2), f(0.9), f(0.95), f(1e-8), f(0.1), f(0.1), f(0.05), f(0.5), 1, OF._s()), "adam")
+    P, M, V, G = (t[sl].double() for t in (*keep[:3], g))
+    G = G * 0.5
+    M, V = 0.9 * M + 0.1 * G, 0.95 * V + 0.05 * G * G
+    P = P - (1e-2 / 0.1 * M / (V.sqrt() / 0.05 ** 0.5 + 1e-8) + 1e-2 * 0.1 * P)
+    for have, want in ((p, P), (m, M), (v, V)):
+        _close(have[sl], want, 1e-6, rtol=2e-6)
+    assert torch.equal(out[sl], p[sl].to(dtype))
+    for have, was in zip((p, m, v, out), keep):
+        assert torch.equal(have[:offset], was[:offset]) and torch.equal(have[offset + n:], was[offset + n:])
