@@ -48,21 +48,14 @@ class _WKV6(torch.autograd.Function):
         B, T, C = r.shape
         H, N = ub.shape
         gy = gy.contiguous()
-        gr, gk, gv = torch.empty_like(r), torch.empty_like(r), torch.empty_like(r)
-        grS = torch.empty(B, T, C, dtype=torch.float32, device=r.device)
-        gkG = torch.empty(B, T, C, dtype=torch.float32, device=r.device)
+        gr, gk, gv, gw = torch.empty_like(r), torch.empty_like(r), torch.empty_like(r), torch.empty_like(r)
+        cum = torch.empty(2, B, T, C, dtype=torch.float32, device=r.device)
         gu_part = torch.empty(B, H, N, dtype=torch.float32, device=r.device)
         rc = native.lib().neox_wkv6_bwd(B, T, C, H, native.ptr(r), native.ptr(k), native.ptr(v), native.ptr(ew),
-                                        native.ptr(ub), native.ptr(gy), native.ptr(gr), native.ptr(gk),
-                                        native.ptr(gv), native.ptr(grS), native.ptr(gkG), native.ptr(gu_part),
+                                        native.ptr(ub), native.ptr(gy), native.ptr(gr), native.ptr(gk), native.ptr(gv),
+                                        native.ptr(gw), native.ptr(cum), native.ptr(gu_part),
                                         ctypes.c_void_p(native.stream_ptr()))
         native.check(rc, "neox_wkv6_bwd")
-        # d_t * dL/dd_t = sum_{s>t} r_s grS_s - sum_{s>=t} k_s gkG_s   (reverse cumulative sums over time)
-        a = r.float() * grS
-        b = k.float() * gkG
-        ra = torch.flip(torch.cumsum(torch.flip(a, [1]), 1), [1]) - a
-        rb = torch.flip(torch.cumsum(torch.flip(b, [1]), 1), [1])
-        gw = ((ra - rb) * ew).to(r.dtype)
         return gr, gk, gv, gw, gu_part.sum(0).to(ctx.u_dtype)
 
 

@@ -1214,3 +1214,25 @@ def test_adam_shards_of_any_alignment(n, offset, dtype):
     assert torch.equal(out[sl], p[sl].to(dtype))
     for have, was in zip((p, m, v, out), keep):
         assert torch.equal(have[:offset], was[:offset]) and torch.equal(have[offset + n:], was[offset + n:])
+
+
+@pytest.mark.parametrize("B,T,H,N", [(1, 1, 1, 32), (2, 16, 2, 64), (1, 65, 3, 64), (2, 200, 2, 128), (1, 700, 2, 32),
+                                     (300, 130, 4, 32)])
+def test_wkv6_groups_match_reference_scan(B, T, H, N):
+    """Edges of the staged groups of eight steps (one step, whole groups, a group and one step, fewer groups than pieces of a
+    state row, more heads than the machine holds) against the sequential recurrence in fp32.  bf16 results: half an ulp (2^-9) of the value plus the
+    fp32 sums' error, which scales with the largest result."""
+    from gpt_neox_b200.ops import wkv6 as W
+    torch.manual_seed(T)
+    C = H * N
+    mk = lambda scale=1.0: (torch.randn(B, T, C, device=DEV) * scale).to(torch.bfloat16).requires_grad_()
+    r, k, v, w = mk(), mk(0.5), mk(), mk(1.5)
+    u = (torch.randn(H, N, device=DEV) * 0.3).to(torch.bfloat16).requires_grad_()
+    y = W.wkv6(r, k, v, w, u)
+    g = torch.randn_like(y)
+    got = torch.autograd.grad(y, (r, k, v, w, u), g)
+    ref_in = [t.detach().float().requires_grad_() for t in (r, k, v, w, u)]
+    yr = W.wkv6_ref(*ref_in)
+    want = torch.autograd.grad(yr, ref_in, g.float(), allow_unused=True)       # one step uses no decay
+    for a, b_ in zip([y, *got], [yr, *[torch.zeros_like(t) if w_ is None else w_ for t, w_ in zip(ref_in, want)]]):
+        _close(a, b_, 1e-3 + 2e-3 * b_.abs().max().item(), rtol=4e-3)
