@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "launch.cuh"
 #include "neox_b200.h"
 
 namespace {
@@ -92,6 +93,8 @@ __global__ void __launch_bounds__(DA_THREADS) decode_attn_kernel(const DecodePar
     const int csize = (int)cluster.num_blocks(), crank = (int)cluster.block_rank();
     const int h = blockIdx.y, bi = blockIdx.z, rep = p.hq / p.hkv, hk = h / rep;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    launch::let_successor_start();
+    launch::wait_for_predecessor();
     // the host keeps the position inside the cache; the clamp only bounds what a wrong one could touch
     const int n = p.pos ? (int)min(max(*p.pos, 0ll), (long long)p.cap - 1) : p.n;
     const float cs = p.scale * LOG2E;
@@ -219,21 +222,6 @@ __global__ void __launch_bounds__(DA_THREADS) decode_attn_kernel(const DecodePar
     }
 }
 
-template <int D, bool H16>
-int launch(const DecodeParams& p, int csize, cudaStream_t s) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(csize, p.hq, p.b);
-    cfg.blockDim = dim3(DA_THREADS);
-    cfg.stream = s;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = csize;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, decode_attn_kernel<D, H16>, p) == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
-}
-
 }  // namespace
 
 // strides: element strides (batch, head) of q, k, v.  n: rows cached so far (the new row's index), or with `pos` an upper
@@ -252,7 +240,10 @@ extern "C" int neox_decode_attn(const void* q, const void* k, const void* v, voi
     int csize = 1;
     while (csize < 8 && (long long)b * hq * csize < neox_sm_count() && keys > 128 * csize) csize *= 2;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define DA_CASE(D_) case D_: return h16 ? launch<D_, true>(p, csize, s) : launch<D_, false>(p, csize, s);
+#define DA_CASE(D_)  \
+    case D_:         \
+        return launch::overlapped(h16 ? decode_attn_kernel<D_, true> : decode_attn_kernel<D_, false>, dim3(csize, hq, b), \
+                                  dim3(DA_THREADS), csize, s, p);
     switch (d) {
         DA_CASE(64)
         DA_CASE(96)

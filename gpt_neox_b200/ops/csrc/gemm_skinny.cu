@@ -3,7 +3,8 @@
 // This is the linear layer of a decoding step: W is read once and dominates (2 N K bytes against 2 M K + 2 M N), so the
 // kernel is a stream over W bound by HBM, and what counts is how many bytes are in flight.  The 128 x 256-tile tcgen05
 // kernel puts N / 256 CTAs on the machine (8 of 148 SMs for N = 2048), each walking all of K behind a 4-stage ring:
-// 29 us per call in a 1.4B model's decoding step at batch 4 and 8, 18.5 us at hidden 1024, batch 1; here 13 and 8.7 us.
+// 29 us per call in a 1.4B model's decoding step at batch 4 and 8, 18.5 us at hidden 1024, batch 1; here 6.6 and 4.2 us in
+// a replayed graph (15 and 3.8 us of bytes for the four products of a layer).
 //
 // Split: a CTA owns 16 rows of W (one mma tile), its 8 warps take the 64-wide k-blocks in turn and, when N / 16 CTAs do
 // not fill the machine, a cluster of 2 to 8 CTAs splits K further.  Partial sums meet in shared memory (distributed
@@ -12,9 +13,15 @@
 // permutation, so the 8 consecutive elements a lane holds serve as its fragments of two m16n8k16 products, with no pass
 // through shared memory.  The tensor-core products only keep the arithmetic out of the way of the loads (at 16 rows
 // packed-fp32 FMAs would already take longer than the bytes); a tcgen05 tile would be 1 / 4 to 1 / 128 full.
+//
+// A CTA asks for its whole share of W in L2 before it waits for the kernel in front (launch.cuh), so registers do not have
+// to hold what is in flight; they are kept few instead, and four CTAs share an SM.  The four products of a layer, batch 1,
+// replayed, hidden 1024 / 2048 / 4096: 29.9 / 42.4 / 100 us with two CTAs an SM and plain launches, 27.7 / 39.7 / 91 with
+// the early request, 16.7 / 26.1 / 83 with four CTAs as well (3.8 / 15.1 / 60.5 of bytes).
 #include <cooperative_groups.h>
 
 #include "gemm_common.cuh"
+#include "launch.cuh"
 #include "neox_b200.h"
 
 namespace {
@@ -58,7 +65,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 
 // NT: groups of 8 rows of X.  U: k-blocks of a warp whose loads are issued together.
 template <bool H16, int NT, int U>
-__global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_kernel(const SkinnyParams p) {
+__global__ void __launch_bounds__(SK_THREADS, NT == 4 ? 2 : 4) gemm_skinny_kernel(const SkinnyParams p) {
     __shared__ float part[SK_WARPS][NT * 8][SK_ROWS + 1];
     __shared__ float mine[NT * 8][SK_ROWS + 1];
     cg::cluster_group cluster = cg::this_cluster();
@@ -72,6 +79,12 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_kernel(const Skinny
     const char* W1 = W0 + 8 * p.ldw * 2;
     const char* X0 = static_cast<const char*>(p.X) + ((long long)lr * p.ldx + lk) * 2;
     const bool w0 = n0 + lr < N, w1 = n0 + lr + 8 < N;
+    // the weights do not depend on the kernel in front: ask for this CTA's share while that one finishes
+    launch::let_successor_start();
+    if (lane < SK_ROWS && n0 + lane < N)
+        for (int kb = crank * SK_WARPS + warp; kb < nblk; kb += slices)
+            launch::prefetch_l2(static_cast<const char*>(p.W) + ((long long)(n0 + lane) * p.ldw + kb * SK_BK) * 2);
+    launch::wait_for_predecessor();
     float acc[NT][4];
 #pragma unroll
     for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
@@ -157,18 +170,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_kernel(const Skinny
 }
 
 template <bool H16, int NT, int U>
-int launch(const SkinnyParams& p, int tiles, int csize, cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles * csize);
-    cfg.blockDim = dim3(SK_THREADS);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = csize;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<H16, NT, U>, p) == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
+int run(const SkinnyParams& p, int tiles, int csize, cudaStream_t stream) {
+    return launch::overlapped(gemm_skinny_kernel<H16, NT, U>, dim3(tiles * csize), dim3(SK_THREADS), csize, stream, p);
 }
 
 }  // namespace
@@ -193,16 +196,15 @@ extern "C" int neox_gemm_skinny_16(const void* A, const void* B, void* D, int M,
     e.aux = static_cast<const __nv_bfloat16*>(aux); e.ldaux = ldaux;
     e.act = act; e.alpha = alpha; e.vec_ok = 0; e.status = nullptr; e.row_ptrs = nullptr;
     const int tiles = (N + SK_ROWS - 1) / SK_ROWS, nblk = (K + SK_BK - 1) / SK_BK;
-    // Split K over a cluster until there are three CTAs for every SM (two are resident, a third fills the gaps) or every
-    // warp is down to one k-block.
-    const int want = 3 * neox_sm_count();
+    // Split K over a cluster while one wave (four CTAs an SM) still holds them all and no warp runs out of k-blocks.
+    const int wave = 4 * neox_sm_count();
     int csize = 1;
-    while (csize < 8 && tiles * csize < want && nblk >= 2 * csize * SK_WARPS) csize *= 2;
+    while (csize < 8 && tiles * csize * 2 <= wave && nblk >= 2 * csize * SK_WARPS) csize *= 2;
     cudaStream_t s = static_cast<cudaStream_t>(stream_);
 #define SK_LAUNCH(H)                                                  \
-    return M <= 8    ? launch<H, 1, 4>(p, tiles, csize, s)            \
-           : M <= 16 ? launch<H, 2, 2>(p, tiles, csize, s)            \
-                     : launch<H, 4, 1>(p, tiles, csize, s)
+    return M <= 8    ? run<H, 1, 2>(p, tiles, csize, s)            \
+           : M <= 16 ? run<H, 2, 1>(p, tiles, csize, s)            \
+                     : run<H, 4, 1>(p, tiles, csize, s)
     if (h16) SK_LAUNCH(true);
     SK_LAUNCH(false);
 #undef SK_LAUNCH

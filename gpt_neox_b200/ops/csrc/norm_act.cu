@@ -6,6 +6,7 @@
 // Replaces apex fused_layer_norm_cuda / FastLayerNormFN (megatron/model/fused_layer_norm.py:123-153),
 // the TorchScript bias_gelu (activations.py:78-112), the gated-activation glue (transformer.py:190-206)
 // and bias_dropout_add (fused_bias_dropout.py:28-55) of the reference.
+#include "launch.cuh"
 #include "neox_b200.h"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -168,6 +169,8 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
     const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, width = WARP ? 32 : blockDim.x;
     const int first = WARP ? blockIdx.x * ROW_WARPS + (threadIdx.x >> 5) : blockIdx.x;
     const int step = WARP ? gridDim.x * ROW_WARPS : gridDim.x;
+    launch::let_successor_start();
+    launch::wait_for_predecessor();
     typename Vec8<T>::Raw nxt[CACHED ? V : 1];
     auto fetch = [&](int r) {
 #pragma unroll
@@ -586,9 +589,9 @@ int launch_norm_fwd_t(const void* x, const void* gamma, const void* beta, void* 
         constexpr int V = decltype(v)::value;
         constexpr bool WARP = decltype(warp)::value;
         const int blocks = WARP ? (rows + ROW_WARPS - 1) / ROW_WARPS : rows, most = neox_sm_count() * 8;
-        norm_fwd_kernel<T, RMS, V, WARP><<<blocks < most ? blocks : most, WARP ? ROW_WARPS * 32 : cta_threads(cols / 8, V), 0, st>>>(
-            (const T*)x, (const T*)gamma, (const T*)beta, (T*)y, s0, s1, rows, cols, eps);
-        return 0;
+        return launch::overlapped(norm_fwd_kernel<T, RMS, V, WARP>, dim3(blocks < most ? blocks : most),
+                                  dim3(WARP ? ROW_WARPS * 32 : cta_threads(cols / 8, V)), 1, st, (const T*)x, (const T*)gamma,
+                                  (const T*)beta, (T*)y, s0, s1, rows, cols, eps);
     });
 }
 
@@ -597,10 +600,9 @@ int launch_norm_fwd(const void* x, const void* gamma, const void* beta, void* y,
                     int cols, float eps, int dtype, cudaStream_t st) {
     if (cols % 8) return NEOX_ERR_SHAPE;
     if (rows <= 0) return 0;
-    if (dtype == 0) launch_norm_fwd_t<__nv_bfloat16, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
-    else if (dtype == 1) launch_norm_fwd_t<float, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
-    else launch_norm_fwd_t<__half, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
-    return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
+    if (dtype == 0) return launch_norm_fwd_t<__nv_bfloat16, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
+    if (dtype == 1) return launch_norm_fwd_t<float, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
+    return launch_norm_fwd_t<__half, RMS>(x, gamma, beta, y, s0, s1, rows, cols, eps, st);
 }
 
 template <typename T, bool RMS>
