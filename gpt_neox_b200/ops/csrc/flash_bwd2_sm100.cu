@@ -17,6 +17,7 @@
 // bounds these kernels: 128-wide blocks and TMEM-resident P / dS halve the operand traffic of the 64-wide form.
 // The softmax scale of dS is applied once to dK and dQ in the epilogues.  Head sizes 64 / 96 / 128, bf16 or fp16.
 // Replaces the flash-attn 2 backward behind megatron/model/transformer.py:627-744.  Every wait is bounded.
+#include "flash_order.cuh"
 #include "sm100_ptx.cuh"
 #include "neox_b200.h"
 #include <cuda_fp16.h>
@@ -42,6 +43,7 @@ struct Bwd2Params {
     void *dq, *dk, *dv;  // [s, b, h, d] views of 16-bit elements; element strides of (s, b, h) below
     long long dq_s[3], dk_s[3], dv_s[3];
     int* status;
+    TileOrder kv_order, q_order;
 };
 
 template <bool FP16>
@@ -165,8 +167,10 @@ flash_bwd2_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kv0 = blockIdx.x * 128;
-    const int bb = blockIdx.y / p.hkv, hk = blockIdx.y % p.hkv;
+    int rank, head;
+    pick_tile(p.kv_order, rank, head);
+    const int kv0 = rank * 128;                 // early keys are attended to by the most rows
+    const int bb = head / p.hkv, hk = head % p.hkv;
     const int G = p.hq / p.hkv;
     const int off = p.sk - p.sq;
     int q_lo = 0, q_hi = p.sq;       // query rows that can attend to this key tile
@@ -439,9 +443,11 @@ flash_bwd2_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q_tile = gridDim.x - 1 - blockIdx.x;
+    int rank, head;
+    pick_tile(p.q_order, rank, head);
+    const int q_tile = p.q_order.tiles - 1 - rank;
     const int q0 = q_tile * 128;
-    const int bb = blockIdx.y / p.hq, h = blockIdx.y % p.hq;
+    const int bb = head / p.hq, h = head % p.hq;
     const int hk = h / (p.hq / p.hkv);
     const int off = p.sk - p.sq;
     int kv_end = p.sk, kv_begin = 0;
@@ -664,11 +670,11 @@ int launch_bwd2(const CUtensorMap* t, const Bwd2Params& p, cudaStream_t st) {
             return NEOX_ERR_LAUNCH;
         attr = true;
     }
-    dim3 gkv((p.sk + 127) / 128, p.b * p.hkv);
-    flash_bwd2_dkv_kernel<D, FP16><<<gkv, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
+    const long long gkv = (long long)p.kv_order.tiles * p.kv_order.heads, gq = (long long)p.q_order.tiles * p.q_order.heads;
+    if (gkv > 0x7fffffff || gq > 0x7fffffff) return NEOX_ERR_SHAPE;
+    flash_bwd2_dkv_kernel<D, FP16><<<(int)gkv, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
     if (cudaGetLastError() != cudaSuccess) return NEOX_ERR_LAUNCH;
-    dim3 gq((p.sq + 127) / 128, p.b * p.hq);
-    flash_bwd2_dq_kernel<D, FP16><<<gq, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
+    flash_bwd2_dq_kernel<D, FP16><<<(int)gq, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
@@ -722,6 +728,8 @@ extern "C" int neox_flash_bwd2_strided(const void* q, const void* k, const void*
         p.dk_s[i] = g_s[3 + i];
         p.dv_s[i] = g_s[6 + i];
     }
+    p.kv_order = tile_order((sk + 127) / 128, b * hkv, 4ll * sq * d * (hq / hkv));      // its heads' queries and gradients
+    p.q_order = tile_order((sq + 127) / 128, b * hq, 4ll * sk * d / (hq / hkv));
     p.status = neox_status_word();
     if (!p.status) return NEOX_ERR_DRIVER;
     if (d == 64) return h16 ? launch_bwd2<64, true>(t, p, st) : launch_bwd2<64, false>(t, p, st);

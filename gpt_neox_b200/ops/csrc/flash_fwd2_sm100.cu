@@ -21,6 +21,7 @@
 // attention (kv head = q head / (hq / hkv)), bottom-right aligned causal mask when sq < sk.
 //
 // Replaces the flash-attn 2 calls of megatron/model/transformer.py:627-744.  Every wait is bounded.
+#include "flash_order.cuh"
 #include "sm100_ptx.cuh"
 #include "neox_b200.h"
 #include <cuda_fp16.h>
@@ -44,6 +45,7 @@ struct Fwd2Params {
     void* out;             // [sq, b, hq, d] contiguous, 16-bit
     float* lse;            // [b, hq, sq]
     int* status;
+    TileOrder order;
 };
 
 template <int D>
@@ -164,8 +166,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q_pair = gridDim.x - 1 - blockIdx.x;      // heavy (late) query tiles first
-    const int bh = blockIdx.y;
+    int rank, bh;
+    pick_tile(p.order, rank, bh);
+    const int q_pair = p.order.tiles - 1 - rank;        // heavy (late) query tiles first
     const int bb = bh / p.hq, h = bh % p.hq;
     const int hk = h / (p.hq / p.hkv);
     const int off = p.sk - p.sq;
@@ -526,8 +529,9 @@ int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
             return NEOX_ERR_LAUNCH;
         attr = true;
     }
-    dim3 grid((p.sq + 2 * BM - 1) / (2 * BM), p.b * p.hq);
-    flash_fwd2_kernel<D, FP16><<<grid, THREADS, Cfg2<D>::SMEM, st>>>(tq, tk, tv, p);
+    const long long grid = (long long)p.order.tiles * p.order.heads;
+    if (grid > 0x7fffffff) return NEOX_ERR_SHAPE;
+    flash_fwd2_kernel<D, FP16><<<(int)grid, THREADS, Cfg2<D>::SMEM, st>>>(tq, tk, tv, p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
@@ -556,6 +560,7 @@ extern "C" int neox_flash_fwd2(const void* q, const void* k, const void* v, void
     p.causal = causal; p.window = window; p.slopes = slopes;
     p.out = out;
     p.lse = lse;
+    p.order = tile_order((sq + 2 * BM - 1) / (2 * BM), b * hq, 4ll * sk * d / (hq / hkv));      // its keys and values
     p.status = neox_status_word();
     if (!p.status) return NEOX_ERR_DRIVER;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
