@@ -220,6 +220,16 @@ EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
+// cuTensorMapEncodeTiled wants a current context.  A thread whose first CUDA work this is (autograd's, in a backward pass that
+// begins with one of these products) has none until a runtime call binds the device's primary one: bind it and ask again.
+template <typename Encode>
+CUresult with_context(Encode encode) {
+    CUresult r = encode();
+    int dev = 0;
+    if (r != CUDA_SUCCESS && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+    return r;
+}
+
 struct MapKey {
     const void* ptr;
     unsigned long long d0, d1, ld;
@@ -265,9 +275,11 @@ static int make_tmap_2d(CUtensorMap* out, const void* ptr, unsigned long long d0
     cuuint64_t strides[1] = {ld * esize};
     cuuint32_t box[2] = {b0, b1};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(out, esize == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                     const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = with_context([&] {
+        return enc(out, esize == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                   const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    });
     if (r != CUDA_SUCCESS) return NEOX_ERR_TMAP;
     std::lock_guard<std::mutex> g(g_map_mu);
     if (g_maps.size() > 8192) g_maps.clear();
@@ -300,9 +312,11 @@ int neox_make_tmap_bf16_4d(CUtensorMap* out, const void* ptr, unsigned long long
     // a size-1 dimension may carry any stride; the encoder wants strides that are positive multiples of 16
     for (int i = 0; i < 3; ++i)
         if (strides[i] == 0) strides[i] = 16;
-    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = with_context([&] {
+        return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    });
     return r == CUDA_SUCCESS ? 0 : NEOX_ERR_TMAP;
 }
 
