@@ -61,16 +61,16 @@ class _VocabParallelCE(torch.autograd.Function):
         tgt = target.reshape(-1).contiguous()
         tp = mpu.get_model_parallel_world_size()
         v0 = mpu.get_model_parallel_rank() * vloc
-        if _k(logits2) and logits2.dtype == torch.bfloat16 and vloc % 8 == 0 and \
-                native.lib().has("neox_ce_online_bf16"):
+        if _k(logits2) and logits2.dtype in (torch.bfloat16, torch.float16) and vloc % 8 == 0 and \
+                logits2.data_ptr() % 16 == 0:
             # one pass over the logits: local (max, sum exp, raw target logit), re-based on the global maximum after
             # the first all-reduce
             rows = logits2.shape[0]
             row_max = torch.empty(rows, dtype=torch.float32, device=logits2.device)
             stats = torch.empty(rows, 2, dtype=torch.float32, device=logits2.device)
-            rc = native.lib().neox_ce_online_bf16(native.ptr(logits2), native.ptr(tgt), native.ptr(row_max),
-                                                  native.ptr(stats), rows, vloc, v0, _s())
-            native.check(rc, "neox_ce_online_bf16")
+            rc = native.lib().neox_ce_online_16(native.ptr(logits2), native.ptr(tgt), native.ptr(row_max),
+                                                native.ptr(stats), rows, vloc, v0, _DT[logits2.dtype], _s())
+            native.check(rc, "neox_ce_online_16")
             local_max = row_max
             if tp > 1:
                 row_max = local_max.clone()
