@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(SK_THREADS, NT == 4 ? 2 : 4) gemm_skinny_kerne
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
                     x[i][half][t] = k + lk < K && t * 8 + lr < M
-                                        ? __ldg(reinterpret_cast<const uint4*>(X0 + (t * 8 * p.ldx + k) * 2))
+                                        ? launch::load_16(X0 + (t * 8 * p.ldx + k) * 2)
                                         : zero;
             }
         }

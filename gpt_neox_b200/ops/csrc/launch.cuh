@@ -16,6 +16,15 @@ __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcon
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// 16 bytes that the kernel in front may have written, read after the wait: a coherent load.  (Read-only loads, which the
+// compiler also makes of `const __restrict__` pointers, assume data that is constant for the kernel's whole life; a kernel that
+// starts early lives through its predecessor's writes.)
+__device__ __forceinline__ uint4 load_16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // cluster: thread blocks per cluster along x (1: none)
 template <typename... Params, typename... Args>
 int overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, int cluster, cudaStream_t stream, Args... args) {

@@ -104,6 +104,16 @@ struct Vec8<float> {
     }
 };
 
+// 8 elements that the kernel in front may have written (see launch.cuh)
+template <typename T>
+__device__ __forceinline__ typename Vec8<T>::Raw coherent_load(const T* p) {
+    typename Vec8<T>::Raw r;
+    uint4* w = reinterpret_cast<uint4*>(&r);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(r) / 16); ++i) w[i] = launch::load_16(reinterpret_cast<const uint4*>(p) + i);
+    return r;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -161,7 +171,7 @@ __device__ __forceinline__ float row_sum(float v, float (&red)[32]) {
 
 template <typename T, bool RMS, int V, bool WARP>
 __global__ void __launch_bounds__(WARP ? ROW_WARPS * 32 : CTA_THREADS)
-norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
+norm_fwd_kernel(const T* x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
                 float* __restrict__ stat0, float* __restrict__ stat1, int rows, int cols, float eps) {
     __shared__ float red0[32], red1[32];
     constexpr bool CACHED = V > 0;
@@ -176,7 +186,7 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
 #pragma unroll
         for (int j = 0; j < V; ++j) {
             const int c = tid + j * width;
-            if (c < nvec) nxt[j] = Vec8<T>::raw_load(x + (size_t)r * cols + c * 8);
+            if (c < nvec) nxt[j] = coherent_load(x + (size_t)r * cols + c * 8);
         }
     };
     if (CACHED && first < rows) fetch(first);
@@ -199,7 +209,7 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
         } else {
             for (int c = tid; c < nvec; c += width) {
                 float t[8];
-                Vec8<T>::load(xr + c * 8, t);
+                Vec8<T>::unpack(coherent_load(xr + c * 8), t);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) s += RMS ? t[i] * t[i] : t[i];
             }
@@ -227,7 +237,7 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
             } else {
                 for (int c = tid; c < nvec; c += width) {
                     float t[8];
-                    Vec8<T>::load(xr + c * 8, t);
+                    Vec8<T>::unpack(coherent_load(xr + c * 8), t);
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const float d = t[i] - mean;
@@ -259,7 +269,7 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* _
         } else {
             for (int c = tid; c < nvec; c += width) {
                 float t[8];
-                Vec8<T>::load(xr + c * 8, t);
+                Vec8<T>::unpack(coherent_load(xr + c * 8), t);
                 emit(c, t);
             }
         }
