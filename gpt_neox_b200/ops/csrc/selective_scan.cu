@@ -16,8 +16,8 @@
 // arithmetic around it; the bytes are a tenth of that.  One thread per channel walking all of time serially, as this
 // file did before, left most SMs without a block (6144 channels = 48 blocks forward, 96 of two warps backward) and paid
 // the latency of every step: 1987 us forward, 7232 us backward at b 4, l 2048, d 1536.  The chunked form computes the
-// exponentials twice and has 64 times the threads: 181 us forward (state 67, combine 10, output 104) and 588 us backward
-// (adjoint 82, combine 15, gradient 491).  Exponentials alone would take 45 us a pass.
+// exponentials twice and has 64 times the threads: 181 us forward (state 67, combine 10, output 104) and 514 us backward
+// (adjoint 82, combine 15, gradient 417).  Exponentials alone would take 45 us a pass.
 #include "neox_b200.h"
 #include <cuda_bf16.h>
 
@@ -261,25 +261,28 @@ scan_adjoint_kernel(const bf16* __restrict__ dt, const float* __restrict__ A, co
 
 // ------------------------------------------------------------------ backward: gradients of one chunk
 // A block takes one chunk of 64 channels; four threads share a channel and hold four states each (lane = 8 * state group
-// + channel of the warp), so that the states and decays of eight steps fit into registers: a sub-chunk of eight steps is
+// + channel of the warp), so that the states and decays of a few steps fit into registers: a sub-chunk of four steps is
 // recomputed forwards from its start state and walked backwards at once, and no per-step state leaves the registers.
+// Sub-chunks of four and results written over the staged operands keep it to 80 registers and 68 KB, three blocks on an SM:
+// 491 us with sub-chunks of eight on two blocks, 417 us so (b 4, l 2048, d 1536).
 // Per-element quantities that do not depend on the state index (softplus, SiLU) are computed once and shared through
 // shared memory.  Sums over the states of a channel and over the channels of a warp are reduced "transposed" (every
 // shuffle step halves the number of values a lane carries): 3 + 7 shuffles per step instead of 6 + 24.
 constexpr int GCH = 64;                       // channels per block
 constexpr int GTH = GCH * 4;                  // threads per block
-constexpr int NSUB = CHUNK / GROUP;
+constexpr int GSTEP = 4;                      // steps per sub-chunk
+constexpr int NSUB = CHUNK / GSTEP;
 
 struct GradSmem {
-    float delta[CHUNK][GCH], u[CHUNK][GCH], gy[CHUNK][GCH];       // staged per-element inputs
-    float y[CHUNK][GCH], sa[CHUNK][GCH], sb[CHUNK][GCH];          // sums over the states
+    // staged per-element inputs; once a step has been walked, in their places the step's sums over the states: gd * a, g * B, y
+    float delta[CHUNK][GCH], u[CHUNK][GCH], gy[CHUNK][GCH];
     alignas(16) float B[CHUNK][NS];
     alignas(16) float C[CHUNK][NS];
     float start[NSUB][4][GTH];                                    // state at the start of every sub-chunk
-    float red[GTH / 32][GROUP][32];                               // dB | dC partial sums per warp
+    float red[2][GTH / 32][GSTEP][32];                            // dB | dC partial sums per warp, of two sub-chunks in turn
 };
 
-__global__ void __launch_bounds__(GTH, 2)
+__global__ void __launch_bounds__(GTH, 3)
 scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const float* __restrict__ A,
                  const float* __restrict__ B, const float* __restrict__ C, const float* __restrict__ D,
                  const bf16* __restrict__ z, const float* __restrict__ bias, const float* __restrict__ ckpt,
@@ -335,8 +338,8 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
         for (int j = 0; j < 4; ++j) sm.start[sub][j][tid] = h[j];
         if (sub == NSUB - 1) break;
 #pragma unroll
-        for (int i = 0; i < GROUP; ++i) {
-            const int s = sub * GROUP + i;
+        for (int i = 0; i < GSTEP; ++i) {
+            const int s = sub * GSTEP + i;
             const float delta = sm.delta[s][cc], du = delta * sm.u[s][cc], d2 = delta * LOG2E;
             const float4 bv = *reinterpret_cast<const float4*>(&sm.B[s][sg * 4]);
             h[0] = exp2f(d2 * a[0]) * h[0] + du * bv.x;
@@ -348,12 +351,12 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
     // ---- sub-chunks from the last to the first: recompute, then walk backwards
 #pragma unroll 1
     for (int sub = NSUB - 1; sub >= 0; --sub) {
-        float hp[GROUP + 1][4], dA[GROUP][4];
+        float hp[GSTEP + 1][4], dA[GSTEP][4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) hp[0][j] = sm.start[sub][j][tid];
 #pragma unroll
-        for (int i = 0; i < GROUP; ++i) {
-            const int s = sub * GROUP + i;
+        for (int i = 0; i < GSTEP; ++i) {
+            const int s = sub * GSTEP + i;
             const float delta = sm.delta[s][cc], du = delta * sm.u[s][cc], d2 = delta * LOG2E;
             const float4 bv = *reinterpret_cast<const float4*>(&sm.B[s][sg * 4]);
             const float bj[4] = {bv.x, bv.y, bv.z, bv.w};
@@ -364,8 +367,8 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
             }
         }
 #pragma unroll
-        for (int i = GROUP - 1; i >= 0; --i) {
-            const int s = sub * GROUP + i;
+        for (int i = GSTEP - 1; i >= 0; --i) {
+            const int s = sub * GSTEP + i;
             const float delta = sm.delta[s][cc], du = delta * sm.u[s][cc], gy = sm.gy[s][cc];
             const float4 bv = *reinterpret_cast<const float4*>(&sm.B[s][sg * 4]);
             const float4 cv = *reinterpret_cast<const float4*>(&sm.C[s][sg * 4]);
@@ -391,7 +394,8 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
                 // groups 0, 1: exchange y against sa; groups 2, 3: sb (group 3's result is not used)
                 const float r = __shfl_xor_sync(0xffffffffu, odd ? k0 : (hi ? k0 : k1), 8);
                 const float v = (odd ? (hi ? k0 : k1) : k0) + r;
-                if (sg < 3) (sg == 0 ? sm.y : sg == 1 ? sm.sa : sm.sb)[s][cc] = v;
+                __syncwarp();               // every lane has read what this replaces; no other warp uses these channels
+                if (sg < 3) (sg == 0 ? sm.gy : sg == 1 ? sm.delta : sm.u)[s][cc] = v;
             }
             // over the eight channels of the warp (lane bits 0 .. 2): every lane ends with one of pb[0..3], pc[0..3]
             {
@@ -403,24 +407,23 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
                 float r0 = (b1 ? q[2] : q[0]) + __shfl_xor_sync(0xffffffffu, b1 ? q[0] : q[2], 2);
                 float r1 = (b1 ? q[3] : q[1]) + __shfl_xor_sync(0xffffffffu, b1 ? q[1] : q[3], 2);
                 const float v = (b0 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, b0 ? r0 : r1, 1);
-                sm.red[warp][i][(b2 ? 16 : 0) + sg * 4 + (lane & 3)] = v;
+                sm.red[sub & 1][warp][i][(b2 ? 16 : 0) + sg * 4 + (lane & 3)] = v;
             }
         }
-        __syncthreads();
-        {
-            const int i = tid >> 5, s = sub * GROUP + i;        // 8 steps x 32 sums = one per thread
+        __syncthreads();                    // (the other buffer's sums were read before this barrier was reached)
+        if (warp < GSTEP) {
+            const int s = sub * GSTEP + warp;
             float v = 0.f;
 #pragma unroll
-            for (int w = 0; w < GTH / 32; ++w) v += sm.red[w][i][lane];
+            for (int w = 0; w < GTH / 32; ++w) v += sm.red[sub & 1][w][warp][lane];
             if (s < steps) atomicAdd((lane < 16 ? gB : gC) + b * st.gsb + (t0 + s) * st.gst + (lane & 15), v);
         }
-        __syncthreads();
     }
     if (live) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) atomicAdd(gA + (size_t)c * NS + sg * 4 + j, ga[j]);
     }
-    // ---- per-element gradients (the last __syncthreads() above made the state sums visible)
+    // ---- per-element gradients (the last __syncthreads() above made the sums over the states visible)
     {
         const int ce = tid % GCH, ch = c0 + ce;
         float gDc = 0.f, gbc = 0.f;
@@ -430,21 +433,22 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
             for (int i = 0; i < CHUNK / 4; ++i) {
                 const int s = tid / GCH + 4 * i;
                 if (s >= steps) break;
-                const float uv = sm.u[s][ce], gy = sm.gy[s][ce], sb = sm.sb[s][ce];
+                const float uv = __bfloat162float(u[b * st.ub + (t0 + s) * st.ut + ch]);
                 const float x = __bfloat162float(dt[b * st.db + (t0 + s) * st.dt + ch]) + bc;
                 const float zv = __bfloat162float(z[b * st.zb + (t0 + s) * st.zt + ch]);
                 const float go = __bfloat162float(gout[b * st.ob + (t0 + s) * st.ot + ch]);
-                const float sz = sigmoid_f(zv);
-                const float g_dt = (sm.sa[s][ce] + uv * sb) * sigmoid_f(x);             // softplus'
+                const float sz = sigmoid_f(zv), gy = go * zv * sz, sb = sm.u[s][ce];
+                const float g_dt = (sm.delta[s][ce] + uv * sb) * sigmoid_f(x);          // softplus'
                 gDc += gy * uv;
                 gbc += g_dt;
                 gz[b * st.gzb + (t0 + s) * st.gzt + ch] =
-                    __float2bfloat16(go * (Dc * uv + sm.y[s][ce]) * sz * (1.f + zv * (1.f - sz)));
-                gu[b * st.gub + (t0 + s) * st.gut + ch] = __float2bfloat16(gy * Dc + sm.delta[s][ce] * sb);
+                    __float2bfloat16(go * (Dc * uv + sm.gy[s][ce]) * sz * (1.f + zv * (1.f - sz)));
+                gu[b * st.gub + (t0 + s) * st.gut + ch] = __float2bfloat16(gy * Dc + softplus_f(x) * sb);
                 gdt[b * st.gdb + (t0 + s) * st.gdt + ch] = __float2bfloat16(g_dt);
             }
         }
-        float* red = &sm.red[0][0][0];
+        __syncthreads();                    // the last sub-chunk's sums have been read
+        float* red = &sm.red[0][0][0][0];
         red[tid] = gDc;
         red[GTH + tid] = gbc;
         __syncthreads();
