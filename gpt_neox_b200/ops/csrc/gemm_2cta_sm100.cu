@@ -32,11 +32,17 @@ using namespace gemm;
 
 namespace {
 
-constexpr int STAGES2 = 6;
-constexpr int BN_HALF = BN / 2;                       // B columns staged by one CTA
-constexpr int A2_STAGE_BYTES = BM * BK * 2;           // 16 KB: 128 rows x 128 bytes of K
-constexpr int B2_STAGE_BYTES = BN_HALF * BK * 2;      // 16 KB
-constexpr int SMEM2_BYTES = STAGES2 * (A2_STAGE_BYTES + B2_STAGE_BYTES) + 256 + 1024;
+// TN: columns of a tile, 256 or 192; the narrower ones are taken where they fill the last round of tiles better (see
+// narrow_tiles below).
+template <int TN>
+struct PairTile {
+    static constexpr int STAGES = TN == 256 ? 6 : 7;
+    static constexpr int HALF = TN / 2;                           // B columns staged by one CTA
+    static constexpr int A_BYTES = BM * BK * 2;                   // 16 KB: 128 rows x 128 bytes of K
+    static constexpr int B_BYTES = HALF * BK * 2;                 // 16 or 12 KB
+    static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + 256 + 1024;
+};
+constexpr int NARROW_COST_PERCENT = 92;               // a round of 192-column tiles, and a margin, in rounds of wide ones
 constexpr int GROUP_M2 = 8;                           // 256-row tile rows per L2 group
 
 struct PairScales {
@@ -58,13 +64,16 @@ __device__ __forceinline__ void tile_coords2(int tile, int num_m, int num_n, int
 
 // F8: operands are one-byte floats; a stage row still holds 128 bytes of K (128 elements instead of 64), an MMA
 // consumes 32 of them, and an MN-major swizzle row covers 128 elements of the MN dimension instead of 64.
-template <bool F8>
+template <bool F8, int TN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
                  const PairScales x) {
     constexpr int BKE = F8 ? 128 : 64;                // elements of K per stage
     constexpr int MNC = F8 ? 128 : 64;                // elements per MN-major chunk
     constexpr int CHUNK_BYTES = MNC * BKE * (F8 ? 1 : 2);
+    constexpr int STAGES2 = PairTile<TN>::STAGES, BN_HALF = PairTile<TN>::HALF, A2_STAGE_BYTES = PairTile<TN>::A_BYTES,
+                  B2_STAGE_BYTES = PairTile<TN>::B_BYTES;
+    static_assert(TN == 256 || TN == 192, "tile widths that were built and measured");
     constexpr int KSTEPS = 4;                         // MMAs per stage: 32 bytes of K each
 
     extern __shared__ uint8_t smem_raw[];
@@ -109,7 +118,7 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const uint32_t tmem_base = *tmem_slot;
 
     const int num_m = (p.M + 2 * BM - 1) / (2 * BM);
-    const int num_n = (p.N + BN - 1) / BN;
+    const int num_n = (p.N + TN - 1) / TN;
     const int ntiles = num_m * num_n;
     const int nk = (p.K + BKE - 1) / BKE;
 
@@ -123,7 +132,7 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 int m_blk, n_blk;
                 tile_coords2(tile, num_m, num_n, x.group_m, m_blk, n_blk);
                 const int m0 = m_blk * 2 * BM + (int)rank * BM;
-                const int n0 = n_blk * BN + (int)rank * BN_HALF;
+                const int n0 = n_blk * TN + (int)rank * BN_HALF;
                 for (int kb = 0; kb < nk; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1)) {
                         atomicExch(p.status, 121);
@@ -157,8 +166,8 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (leader CTA only)
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = F8 ? make_idesc_f8(2 * BM, BN, p.a_mn, p.b_mn, x.a_fmt, x.b_fmt)
-                                      : make_idesc_16(2 * BM, BN, p.a_mn, p.b_mn, p.h16);
+            const uint32_t idesc = F8 ? make_idesc_f8(2 * BM, TN, p.a_mn, p.b_mn, x.a_fmt, x.b_fmt)
+                                      : make_idesc_16(2 * BM, TN, p.a_mn, p.b_mn, p.h16);
             // operand descriptors: constant upper half; lower half = stage base + k-step offset (16-byte units).
             // K-major: the next 32 bytes of K lie 32 bytes along the swizzled row; MN-major: they are the next
             // 16 (bf16) or 32 (fp8) rows of 128 bytes, with chunks of the MN dimension CHUNK_BYTES apart.
@@ -179,7 +188,7 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     break;
                 }
                 tc_fence_after();
-                const uint32_t tmem_d = tmem_base + buf * BN;
+                const uint32_t tmem_d = tmem_base + buf * 256;
                 for (int kb = 0; kb < nk; ++kb) {
                     if (!mbar_wait(&full[stage], phase)) {
                         atomicExch(p.status, 123);
@@ -225,10 +234,10 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             tc_fence_after();
             const int row = m_blk * 2 * BM + (int)rank * BM + q * 32 + lane;
-            const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * BN;
+            const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + buf * 256;
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                const int col0 = n_blk * BN + c * 32;
+            for (int c = 0; c < TN / 32; ++c) {
+                const int col0 = n_blk * TN + c * 32;
                 if (col0 >= p.N) break;  // warp-uniform
                 uint32_t r[32];
                 tmem_ld_32x32(taddr + c * 32, r);
@@ -252,11 +261,11 @@ gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
 }
 
-template <bool F8>
-int launch_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd,
+template <bool F8, int TN>
+int launch_pair_tn(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd,
                 int a_mn, int b_mn, PairScales x, int d_fp32, const void* bias, const void* add, long long ldadd,
                 int add_fp32, void* preact, long long ldpre, const void* aux, long long ldaux, int act, float alpha,
-                cudaStream_t stream, int h16 = 0) {
+                cudaStream_t stream, int h16) {
     constexpr int BKE = F8 ? 128 : 64, MNC = F8 ? 128 : 64, PITCH = F8 ? 16 : 8;
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda % PITCH) || (ldb % PITCH))
@@ -270,7 +279,7 @@ int launch_pair(const void* A, const void* B, void* D, int M, int N, int K, long
     if (!a_mn) rc = tmap(&tmA, A, K, M, lda, BKE, BM);
     else rc = tmap(&tmA, A, M, K, lda, MNC, BKE);
     if (rc) return rc;
-    if (!b_mn) rc = tmap(&tmB, B, K, N, ldb, BKE, BN_HALF);
+    if (!b_mn) rc = tmap(&tmB, B, K, N, ldb, BKE, PairTile<TN>::HALF);
     else rc = tmap(&tmB, B, N, K, ldb, MNC, BKE);
     if (rc) return rc;
 
@@ -303,17 +312,38 @@ int launch_pair(const void* A, const void* B, void* D, int M, int N, int K, long
     x.group_m = group_m;
     static bool attr_set = false;     // one per instantiation
     if (!attr_set) {
-        if (cudaFuncSetAttribute(gemm_2cta_kernel<F8>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES) !=
+        if (cudaFuncSetAttribute(gemm_2cta_kernel<F8, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairTile<TN>::SMEM) !=
             cudaSuccess)
             return NEOX_ERR_LAUNCH;
         attr_set = true;
     }
-    const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (N + BN - 1) / BN;
+    const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (N + TN - 1) / TN;
     int pairs = num_m * num_n;
     const int max_pairs = neox_sm_count() / 2;
     if (pairs > max_pairs) pairs = max_pairs;
-    gemm_2cta_kernel<F8><<<2 * pairs, NUM_THREADS, SMEM2_BYTES, stream>>>(tmA, tmB, p, x);
+    gemm_2cta_kernel<F8, TN><<<2 * pairs, NUM_THREADS, PairTile<TN>::SMEM, stream>>>(tmA, tmB, p, x);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
+}
+
+// Tiles of 192 columns instead of 256?  Work comes in rounds of one tile per pair of SMs, and a round is bound by the operand
+// bytes an SM takes in, 28 KB against 32 KB per k-block: a round of narrow tiles costs about 7 / 8 of a wide one.  So they
+// pay where both take the same number of rounds: 768, 1024 or 2048 columns over a few thousand rows, two rounds that wide
+// tiles fill to 60 %.  Half of 192 columns is no whole number of 64-column chunks, so an MN-major B keeps the wide tiles.
+// With L2 flushed, wide and narrow: 2331 x 2048 x 2048 36.9 and 32.8 us, x 8192 94.2 and 88.1; 5781 x 1024 x 1024 28.7 and
+// 26.6; 8192 x 768 x 768 28.7 and 24.6 (each with some 8 us of launch and event).  128 columns were tried: three rounds of 0.7.
+bool narrow_tiles(int M, int N) {
+    const long long rows = (M + 2 * BM - 1) / (2 * BM), pairs = neox_sm_count() / 2;
+    const long long wide = (rows * ((N + 255) / 256) + pairs - 1) / pairs, narrow = (rows * ((N + 191) / 192) + pairs - 1) / pairs;
+    return narrow * NARROW_COST_PERCENT < wide * 100;
+}
+
+template <bool F8, typename... Args>
+int launch_pair(const void* A, const void* B, void* D, int M, int N, int K, long long lda, long long ldb, long long ldd, int a_mn,
+                int b_mn, Args... args) {
+    if constexpr (!F8) {
+        if (!b_mn && narrow_tiles(M, N)) return launch_pair_tn<F8, 192>(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, args...);
+    }
+    return launch_pair_tn<F8, 256>(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, args...);
 }
 
 }  // namespace
@@ -325,7 +355,7 @@ extern "C" int neox_gemm_bf16_2cta(const void* A, const void* B, void* D, int M,
                                    const void* aux, long long ldaux, int act, float alpha, void* stream_) {
     return launch_pair<false>(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, PairScales{nullptr, nullptr, 0, 0, 0}, d_fp32,
                               bias, add, ldadd, add_fp32, preact, ldpre, aux, ldaux, act, alpha,
-                              static_cast<cudaStream_t>(stream_));
+                              static_cast<cudaStream_t>(stream_), 0);
 }
 
 // Same with the 16-bit type chosen by h16 (0 = bf16, 1 = fp16).
@@ -347,5 +377,5 @@ extern "C" int neox_gemm_fp8_2cta(const void* A, const void* B, void* D, int M, 
     if ((a_fmt | b_fmt) & ~1) return NEOX_ERR_SHAPE;
     return launch_pair<true>(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn,
                              PairScales{inv_scale_a, inv_scale_b, a_fmt, b_fmt, 0}, d_fp32, bias, add, ldadd, add_fp32,
-                             preact, ldpre, aux, ldaux, act, alpha, static_cast<cudaStream_t>(stream_));
+                             preact, ldpre, aux, ldaux, act, alpha, static_cast<cudaStream_t>(stream_), 0);
 }

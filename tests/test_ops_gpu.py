@@ -1273,3 +1273,23 @@ def test_first_cuda_work_of_a_thread(kind):
     assert torch.is_tensor(got[0]), got[0]
     torch.cuda.synchronize()
     assert torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,narrow", [(2331, 2048, 328, True), (5781, 1024, 520, True), (8192, 768, 264, True),
+                                          (4000, 1160, 1000, True), (2331, 6144, 264, False)])
+def test_pair_gemm_tile_widths(M, N, K, narrow, dtype):
+    """Products that fill a round of 256 x 256 tiles poorly take tiles of 192 columns: column counts that are and are not
+    multiples of 192, a last tile whose second half lies outside, ragged rows and contraction, every epilogue.  16-bit
+    results within half an ulp of the fp32 value (sums of K products, error below K 2^-24 of their size)."""
+    torch.manual_seed(M + N)
+    rows = -(-M // 256)
+    assert (-(-rows * -(-N // 192) // 74) * 92 < -(-rows * -(-N // 256) // 74) * 100) == narrow and G.use_pair_kernel(M, N, K)
+    x, w = torch.randn(M, K, device=DEV).to(dtype), torch.randn(N, K, device=DEV).to(dtype)
+    bias, add, s = torch.randn(N, device=DEV).to(dtype), torch.randn(M, N, device=DEV).to(dtype), K ** -0.5
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for kw in ({}, {"bias": bias, "add": add}, {"bias": bias, "act": G.ACT_GELU, "want_preact": True}, {"out_dtype": torch.float32}):
+        got, want = G.gemm(x, w, alpha=s, **kw), G.gemm_ref(x, w, alpha=s, **{"out_dtype": dtype, **kw})
+        for a, b in zip(got, want) if kw.get("want_preact") else [(got, want)]:
+            _close(a, b, 2e-4 if kw.get("out_dtype") == torch.float32 else half_ulp / 4, rtol=2 * half_ulp)
+    assert native.read_status() == 0
