@@ -939,11 +939,6 @@ int neox_rmsnorm_fwd(const void* x, const void* scale, const void* bias, void* y
                      float eps, int dtype, void* stream) {
     return launch_norm_fwd<true>(x, scale, bias, y, nullptr, rinv, rows, cols, eps, dtype, (cudaStream_t)stream);
 }
-int neox_rmsnorm_bwd(const void* g, const void* x, const void* scale, const float* rinv, void* dx, float* dscale,
-                     float* dbias, float* ws, int rows, int cols, float eps, int dtype, void* stream) {
-    return launch_norm_bwd<true>(g, x, scale, nullptr, rinv, dx, dscale, dbias, ws, rows, cols, eps, dtype,
-                                 (cudaStream_t)stream);
-}
 int neox_dgelu_mul(const void* g, const void* pre, void* out, long long n, int dtype, void* stream) {
     return launch_ew<0>(pre, g, nullptr, out, n, 8, dtype, (cudaStream_t)stream);
 }
