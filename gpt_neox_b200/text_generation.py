@@ -11,6 +11,7 @@ other stages; prompts are broadcast from tensor-parallel rank 0.
 from __future__ import annotations
 
 import copy
+import gc
 import json
 import time
 from typing import List, Union
@@ -197,9 +198,18 @@ class GraphDecoder:
                 for _ in range(2):
                     self._forward()
             torch.cuda.current_stream().wait_stream(side)
-            self.graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self.graph):
-                self.logits = self._forward()
+            # A model and its decoders refer to each other, so a decoder of a model that is gone waits for the garbage
+            # collector; were its graph destroyed while this one is captured, the capture would be lost.
+            collecting = gc.isenabled()
+            gc.disable()
+            try:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    self.logits = self._forward()
+                self.graph = graph
+            finally:
+                if collecting:
+                    gc.enable()
         self.graph.replay()
         return self.logits
 
