@@ -156,16 +156,25 @@ def _aligned_rows(t):
 
 
 def _conv_kernel_ok(x, weight, bias):
-    return (x.is_cuda and native.available() and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype
-            and (bias is None or bias.dtype == x.dtype) and weight.shape[1] == 4 and weight.shape[0] % 8 == 0
-            and x.numel() > 0 and x.stride(2) == 1 and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0
-            and x.data_ptr() % 16 == 0)
+    """Do ``x`` ([b, l, d] or [b, l, 2 d]), ``weight`` ([d, 4]) and ``bias`` fit the kernels, which read ``d`` channels of every
+    row of ``x`` and ``d`` contiguous bias elements without asking again?  Whatever does not goes to the library
+    convolution, which takes it or refuses it with a message."""
+    if not (x.is_cuda and native.available() and x.dim() == 3 and weight.dim() == 2):
+        return False
+    b, _, width = x.shape
+    d, taps = weight.shape
+    if bias is not None and not (bias.shape == (d,) and bias.is_contiguous() and bias.dtype == x.dtype
+                                 and bias.device == x.device):
+        return False
+    return (x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype and weight.device == x.device
+            and taps == 4 and d % 8 == 0 and width in (d, 2 * d) and b <= 65535 and x.numel() > 0 and x.stride(2) == 1
+            and x.stride(0) % 8 == 0 and x.stride(1) % 8 == 0 and x.data_ptr() % 16 == 0)
 
 
 def causal_conv1d(x, weight, bias, activation="silu"):
     """Depth-wise causal conv over time for channel-last ``x`` ``[b, l, d]`` (any batch and time strides); ``weight``
     ``[d, w]``.  Width 4 in 16 bits on a GPU: one kernel with bias and SiLU (``csrc/causal_conv.cu``)."""
-    if _conv_kernel_ok(x, weight, bias):
+    if x.shape[-1] == weight.shape[0] and _conv_kernel_ok(x, weight, bias):
         return _CausalConv.apply(x, weight, bias, activation == "silu")[0]
     w = weight.shape[1]
     y = F.conv1d(x.transpose(1, 2), weight.unsqueeze(1), bias, padding=w - 1, groups=weight.shape[0])[..., : x.shape[1]]
@@ -175,7 +184,7 @@ def causal_conv1d(x, weight, bias, activation="silu"):
 
 def causal_conv1d_split(xz, weight, bias):
     """``xz`` ``[b, l, 2 d]`` -> (``silu(conv(first half))``, second half)."""
-    if _conv_kernel_ok(xz, weight, bias):
+    if xz.shape[-1] == 2 * weight.shape[0] and _conv_kernel_ok(xz, weight, bias):
         return _CausalConv.apply(xz, weight, bias, True)
     x, z = xz.chunk(2, dim=-1)
     return causal_conv1d(x, weight, bias), z

@@ -163,3 +163,54 @@ def test_linear_without_gradients_equals_the_recorded_one():
             assert without[1] is None
             with_graph, without = with_graph[0], without[0]
         assert with_graph.requires_grad and not without.requires_grad and torch.equal(with_graph, without)
+
+
+@pytest.fixture
+def conv_routes(monkeypatch):
+    """Lets CPU tensors take the routing of GPU tensors in ``causal_conv1d``: the returned list collects the calls that would
+    have launched the kernel (whose result here is zeros)."""
+    from gpt_neox_b200.ops import native, selective_scan as SS
+    taken = []
+
+    def kernel(xz, weight, bias, silu):
+        taken.append(tuple(xz.shape))
+        return torch.zeros(*xz.shape[:2], weight.shape[0], dtype=xz.dtype), xz[..., weight.shape[0]:]
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True), raising=False)
+    monkeypatch.setattr(native, "available", lambda: True)
+    monkeypatch.setattr(SS._CausalConv, "apply", kernel)
+    return taken
+
+
+@pytest.mark.parametrize("channels,bias,kernel", [
+    (128, 128, True), (128, None, True), (64, 128, False), (256, 128, False), (136, 128, False), (128, 64, False),
+    (128, 256, False), (128, "strided", False), (128, "matrix", False)])
+def test_causal_conv_kernel_takes_only_matching_shapes(conv_routes, channels, bias, kernel):
+    """The kernel reads ``weight.shape[0]`` channels of every row and as many bias elements, whatever the operands hold: a
+    call with other counts is left to the library convolution, which refuses it (a strided bias it accepts)."""
+    from gpt_neox_b200.ops.selective_scan import causal_conv1d
+    x, w = torch.randn(2, 9, channels).bfloat16(), torch.randn(128, 4).bfloat16()
+    if bias == "strided":
+        b = torch.randn(256).bfloat16()[::2]
+    elif bias == "matrix":
+        b = torch.randn(1, 128).bfloat16()
+    else:
+        b = None if bias is None else torch.randn(bias).bfloat16()
+    if kernel or bias == "strided":
+        assert causal_conv1d(x, w, b).shape == (2, 9, 128)
+    else:
+        with pytest.raises(RuntimeError):
+            causal_conv1d(x, w, b)
+    assert bool(conv_routes) == kernel
+
+
+@pytest.mark.parametrize("channels,kernel", [(256, True), (128, False), (264, False), (512, False)])
+def test_causal_conv_split_kernel_takes_only_two_halves(conv_routes, channels, kernel):
+    from gpt_neox_b200.ops.selective_scan import causal_conv1d_split
+    xz, w = torch.randn(2, 9, channels).bfloat16(), torch.randn(128, 4).bfloat16()
+    if kernel:
+        x, z = causal_conv1d_split(xz, w, None)
+        assert x.shape == z.shape == (2, 9, 128)
+    else:
+        with pytest.raises(RuntimeError):
+            causal_conv1d_split(xz, w, None)
+    assert bool(conv_routes) == kernel
