@@ -114,10 +114,15 @@ def stream_ptr() -> int:
 
 def plain_call(*tensors) -> bool:
     """May an operator compute its values directly instead of going through ``torch.autograd.Function`` (20 us of a decoding
-    step's launch)?  Only where that makes no difference: nothing records gradients, no functorch transform, forward-mode
-    level or tracer is active, and the arguments are plain tensors."""
-    if torch.is_grad_enabled() or torch._C._functorch.peek_interpreter_stack() is not None \
-            or forward_ad._current_level >= 0 or torch._C._get_tracing_state() is not None:
+    step's launch)?  Only where that makes no difference: nothing records gradients, and nothing else watches the call."""
+    return not torch.is_grad_enabled() and untransformed(*tensors)
+
+
+def untransformed(*tensors) -> bool:
+    """No functorch transform, forward-mode level or tracer is active, and the arguments are plain tensors: nothing sees more
+    of an operator than its values and its gradients."""
+    if torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0 \
+            or torch._C._get_tracing_state() is not None:
         return False
     for t in tensors:
         if t is not None and type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter:

@@ -125,15 +125,25 @@ class _CausalConv(torch.autograd.Function):
                                                _strides(xz, out), b, l, d, int(silu), int(xz.dtype == torch.float16),
                                                ctypes.c_void_p(native.stream_ptr()))
         native.check(rc, "neox_causal_conv_fwd")
-        ctx.save_for_backward(xz, w, bias)
+        ctx.save_for_backward(xz, weight, bias)
         ctx.silu = silu
         return out, xz[..., d:]
 
     @staticmethod
     def backward(ctx, g, gz):
-        xz, w, bias = ctx.saved_tensors
+        xz, weight, bias = ctx.saved_tensors
         b, l, width = xz.shape
-        d = w.shape[0]
+        d = weight.shape[0]
+        if torch.is_grad_enabled():
+            # create_graph: the gradients are to be differentiated once more, which the kernel's are not
+            leaves = [t for t, wanted in zip((xz, weight, bias), ctx.needs_input_grad) if wanted]
+            out = _library_conv(xz[..., :d], weight, bias, ctx.silu)
+            found = iter(torch.autograd.grad(out, leaves, g, create_graph=True))
+            gxz, gw, gb = (next(found) if wanted else None for wanted in ctx.needs_input_grad[:3])
+            if gxz is not None and width > d:
+                gxz = gxz + torch.cat([torch.zeros_like(g), gz], dim=-1)
+            return gxz, gw, gb, None
+        w = weight.contiguous()
         g = _aligned_rows(g)
         gxz = torch.empty(l, b, width, dtype=xz.dtype, device=xz.device).transpose(0, 1) if xz.stride(0) < xz.stride(1) \
             else torch.empty(b, l, width, dtype=xz.dtype, device=xz.device)
@@ -158,8 +168,9 @@ def _aligned_rows(t):
 def _conv_kernel_ok(x, weight, bias):
     """Do ``x`` ([b, l, d] or [b, l, 2 d]), ``weight`` ([d, 4]) and ``bias`` fit the kernels, which read ``d`` channels of every
     row of ``x`` and ``d`` contiguous bias elements without asking again?  Whatever does not goes to the library
-    convolution, which takes it or refuses it with a message."""
-    if not (x.is_cuda and native.available() and x.dim() == 3 and weight.dim() == 2):
+    convolution, which takes it or refuses it with a message; so do calls under a transform (vmap, forward mode, tracing)
+    that an autograd function would not follow."""
+    if not (x.is_cuda and native.available() and x.dim() == 3 and weight.dim() == 2 and native.untransformed(x, weight, bias)):
         return False
     b, _, width = x.shape
     d, taps = weight.shape
@@ -174,17 +185,21 @@ def _conv_kernel_ok(x, weight, bias):
 def causal_conv1d(x, weight, bias, activation="silu"):
     """Depth-wise causal conv over time for channel-last ``x`` ``[b, l, d]`` (any batch and time strides); ``weight``
     ``[d, w]``.  Width 4 in 16 bits on a GPU: one kernel with bias and SiLU (``csrc/causal_conv.cu``)."""
-    if x.shape[-1] == weight.shape[0] and _conv_kernel_ok(x, weight, bias):
+    if _conv_kernel_ok(x, weight, bias) and x.shape[-1] == weight.shape[0]:
         return _CausalConv.apply(x, weight, bias, activation == "silu")[0]
+    return _library_conv(x, weight, bias, activation == "silu")
+
+
+def _library_conv(x, weight, bias, silu):
     w = weight.shape[1]
     y = F.conv1d(x.transpose(1, 2), weight.unsqueeze(1), bias, padding=w - 1, groups=weight.shape[0])[..., : x.shape[1]]
     y = y.transpose(1, 2)
-    return F.silu(y) if activation == "silu" else y
+    return F.silu(y) if silu else y
 
 
 def causal_conv1d_split(xz, weight, bias):
     """``xz`` ``[b, l, 2 d]`` -> (``silu(conv(first half))``, second half)."""
-    if xz.shape[-1] == 2 * weight.shape[0] and _conv_kernel_ok(xz, weight, bias):
+    if _conv_kernel_ok(xz, weight, bias) and xz.shape[-1] == 2 * weight.shape[0]:
         return _CausalConv.apply(xz, weight, bias, True)
     x, z = xz.chunk(2, dim=-1)
     return causal_conv1d(x, weight, bias), z

@@ -214,3 +214,42 @@ def test_causal_conv_split_kernel_takes_only_two_halves(conv_routes, channels, k
         with pytest.raises(RuntimeError):
             causal_conv1d_split(xz, w, None)
     assert bool(conv_routes) == kernel
+
+
+def test_causal_conv_under_transforms_takes_the_library_path(conv_routes):
+    """vmap, forward mode and tracing follow the library convolution; an autograd function around the kernel they do not."""
+    from torch.autograd import forward_ad
+    from gpt_neox_b200.ops.selective_scan import causal_conv1d
+    x, w, b = torch.randn(3, 2, 9, 16).bfloat16(), torch.randn(16, 4).bfloat16(), torch.randn(16).bfloat16()
+    got = torch.func.vmap(lambda t: causal_conv1d(t, w, b))(x)
+    assert got.shape == x.shape and bool(got.abs().sum() > 0)
+    with forward_ad.dual_level():
+        out = causal_conv1d(forward_ad.make_dual(x[0], torch.ones_like(x[0])), w, b)
+        assert forward_ad.unpack_dual(out).tangent is not None
+    traced = torch.jit.trace(lambda t: causal_conv1d(t, w, b), (x[0],), check_trace=False)
+    assert torch.equal(traced(x[1]), got[1])
+    assert not conv_routes
+    causal_conv1d(x[0], w, b)
+    assert conv_routes
+
+
+@pytest.mark.parametrize("halves", [1, 2])
+def test_causal_conv_gradients_can_be_differentiated(monkeypatch, halves):
+    """``create_graph=True``: second derivatives through the autograd function around the convolution kernel, whose launch is
+    replaced by the library convolution in fp64 here, against finite differences."""
+    from gpt_neox_b200.ops import native, selective_scan as SS
+
+    class Lib:
+        @staticmethod
+        def neox_causal_conv_fwd(x, w, bias, out, strides, b, l, d, silu, *rest):
+            y = torch.nn.functional.conv1d(x[..., :d].transpose(1, 2), w.unsqueeze(1), bias, padding=3, groups=d)[..., :l]
+            out.copy_(torch.nn.functional.silu(y.transpose(1, 2)))
+            return 0
+    monkeypatch.setattr(native, "lib", lambda: Lib)
+    monkeypatch.setattr(native, "ptr", lambda t: t)
+    monkeypatch.setattr(native, "stream_ptr", lambda: 0)
+    torch.manual_seed(0)
+    xz, w, b = (torch.randn(*s, dtype=torch.float64, requires_grad=True) for s in ((2, 5, 3 * halves), (3, 4), (3,)))
+    run = lambda *t: SS._CausalConv.apply(*t, True)[:halves]
+    assert torch.autograd.gradgradcheck(run, (xz, w, b))
+    assert torch.autograd.gradgradcheck(lambda t: SS._CausalConv.apply(t, w.detach(), None, True)[:halves], (xz,))

@@ -1293,3 +1293,27 @@ def test_pair_gemm_tile_widths(M, N, K, narrow, dtype):
         for a, b in zip(got, want) if kw.get("want_preact") else [(got, want)]:
             _close(a, b, 2e-4 if kw.get("out_dtype") == torch.float32 else half_ulp / 4, rtol=2 * half_ulp)
     assert native.read_status() == 0
+
+
+def test_causal_conv_second_derivatives_and_transforms():
+    """What the library convolution offered beside first gradients: second derivatives, vmap and forward mode, in bf16 against
+    the same in fp32 (a few roundings of 2^-8 each)."""
+    from torch.autograd import forward_ad
+    from gpt_neox_b200.ops import selective_scan as SS
+    torch.manual_seed(0)
+    x, w, bs = torch.randn(2, 3, 12, 16, device=DEV), torch.randn(16, 4, device=DEV) * 0.5, torch.randn(16, device=DEV)
+
+    def second(x, w, bs):
+        x, w, bs = (t.detach().requires_grad_() for t in (x, w, bs))
+        y = SS.causal_conv1d(x, w, bs)
+        gx, gw = torch.autograd.grad(y.float().square().sum(), (x, w), create_graph=True)
+        return torch.autograd.grad(gx.float().sum() + gw.float().sum(), (x, w, bs))
+    b16 = lambda *ts: [t.to(torch.bfloat16) for t in ts]
+    for a, b in zip(second(*b16(x[0], w, bs)), second(*(t.float() for t in b16(x[0], w, bs)))):
+        _close(a, b, 0.02 * b.abs().max().item(), rtol=0.02)
+    xb, wb, bb = b16(x, w, bs)
+    plain = torch.stack([SS.causal_conv1d(t, wb, bb) for t in xb])
+    _close(torch.func.vmap(lambda t: SS.causal_conv1d(t, wb, bb))(xb), plain, 2.0 ** -7, rtol=2.0 ** -6)
+    with forward_ad.dual_level():
+        out = SS.causal_conv1d(forward_ad.make_dual(xb[0], torch.ones_like(xb[0])), wb, bb)
+        assert forward_ad.unpack_dual(out).tangent is not None
