@@ -160,9 +160,9 @@ class _CausalConv(torch.autograd.Function):
 
 
 def _aligned_rows(t):
-    """``t`` with unit channel stride and every row on a 16-byte boundary."""
+    """``t`` with unit channel stride and every row on a 16-byte boundary (the channels are a multiple of 8)."""
     ok = t.stride(2) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0
-    return t if ok else t.contiguous()
+    return t if ok else t.clone(memory_format=torch.contiguous_format)      # contiguous() keeps one that starts off a boundary
 
 
 def _conv_kernel_ok(x, weight, bias):

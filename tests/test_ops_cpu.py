@@ -253,3 +253,15 @@ def test_causal_conv_gradients_can_be_differentiated(monkeypatch, halves):
     run = lambda *t: SS._CausalConv.apply(*t, True)[:halves]
     assert torch.autograd.gradgradcheck(run, (xz, w, b))
     assert torch.autograd.gradgradcheck(lambda t: SS._CausalConv.apply(t, w.detach(), None, True)[:halves], (xz,))
+
+
+def test_aligned_rows_moves_a_contiguous_gradient_off_its_odd_start():
+    """A gradient may be any view: contiguous, but starting between two 16-byte boundaries."""
+    from gpt_neox_b200.ops.selective_scan import _aligned_rows
+    flat = torch.randn(2 * 5 * 16 + 24).bfloat16()
+    shift = (-flat.data_ptr() // 2) % 8                          # elements up to the first boundary
+    for off in range(8):
+        t = flat[shift + off: shift + off + 160].view(2, 5, 16)
+        got = _aligned_rows(t)
+        assert torch.equal(got, t) and got.data_ptr() % 16 == 0 and got.stride() == (80, 16, 1)
+        assert (got is t) == (off == 0)
