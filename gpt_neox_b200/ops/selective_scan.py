@@ -50,6 +50,13 @@ def _rows(t, dtype=None):
     return t if t.stride(2) == 1 else t.contiguous()
 
 
+def _like_rows(t):
+    """A new tensor of the shape of ``t``, in its order of batch and time where that leaves the last dimension contiguous, as the
+    kernels write it.  (The dense copy of overlapping windows, strides (s, 1, 1), may put time innermost.)"""
+    new = torch.empty_like(t)
+    return new if new.stride(2) == 1 else torch.empty(t.shape, dtype=t.dtype, device=t.device)
+
+
 def _strides(*ts):
     return (ctypes.c_longlong * (2 * len(ts)))(*[s for t in ts for s in t.stride()[:2]])
 
@@ -63,7 +70,7 @@ class _Scan(torch.autograd.Function):
         Bc, Cc = _rows(B, torch.float32), _rows(C, torch.float32)
         Af, Df, bias = A.float().contiguous(), D.float().contiguous(), dt_bias.float().contiguous()
         nchk = (l + 31) // 32
-        y = torch.empty_like(u)
+        y = _like_rows(u)
         ckpt = torch.empty(b, nchk, n, d, dtype=torch.float32, device=u.device)
         sumd = torch.empty(b, nchk, d, dtype=torch.float32, device=u.device)
         rc = native.lib().neox_selective_scan_fwd(native.ptr(u), native.ptr(dt), native.ptr(Af), native.ptr(Bc),
@@ -82,7 +89,7 @@ class _Scan(torch.autograd.Function):
         b, l, d = u.shape
         n = Af.shape[1]
         gy = _rows(gy)
-        du, ddt, dz = torch.empty_like(u), torch.empty_like(dt), torch.empty_like(z)
+        du, ddt, dz = _like_rows(u), _like_rows(dt), _like_rows(z)
         sums = torch.zeros(d * n + 2 * b * l * n + 2 * d, dtype=torch.float32, device=u.device)
         dA, dB, dC, dD, dbias = sums.split([d * n, b * l * n, b * l * n, d, d])
         dA, dB, dC = dA.view(d, n), dB.view(b, l, n), dC.view(b, l, n)

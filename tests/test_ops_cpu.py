@@ -265,3 +265,14 @@ def test_aligned_rows_moves_a_contiguous_gradient_off_its_odd_start():
         got = _aligned_rows(t)
         assert torch.equal(got, t) and got.data_ptr() % 16 == 0 and got.stride() == (80, 16, 1)
         assert (got is t) == (off == 0)
+
+
+@pytest.mark.parametrize("shape,stride", [((2, 4, 8), (40, 1, 1)), ((2, 8, 4), (40, 2, 1)), ((3, 6, 8), (16, 48, 1)),
+                                          ((3, 6, 8), (0, 0, 1)), ((1, 6, 8), (96, 16, 1)), ((3, 6, 1), (1, 3, 1))])
+def test_scan_results_have_contiguous_channels(shape, stride):
+    """The scan kernels write the last dimension with unit stride, also for an input of overlapping windows, whose dense copy
+    puts time innermost."""
+    from gpt_neox_b200.ops.selective_scan import _like_rows
+    new = _like_rows(torch.zeros(200).as_strided(shape, stride))
+    assert new.shape == shape and (new.stride(2) == 1 or shape[2] == 1)
+    assert new.is_contiguous() or new.transpose(0, 1).is_contiguous()

@@ -1317,3 +1317,22 @@ def test_causal_conv_second_derivatives_and_transforms():
     with forward_ad.dual_level():
         out = SS.causal_conv1d(forward_ad.make_dual(xb[0], torch.ones_like(xb[0])), wb, bb)
         assert forward_ad.unpack_dual(out).tangent is not None
+
+
+def test_selective_scan_on_overlapping_windows():
+    """Windows of one signal (strides (s, 1, 1)) as the input: results and gradients equal those on its copy, bit for bit in
+    the outputs."""
+    from gpt_neox_b200.ops import selective_scan as SS
+    torch.manual_seed(0)
+    b, l, d, n = 2, 40, 64, 16
+    u = torch.randn(b, 256, device=DEV).to(torch.bfloat16).as_strided((b, l, d), (256, 1, 1))
+    dt, z, g = (torch.randn(b, l, d, device=DEV).to(torch.bfloat16) for _ in range(3))
+    B, C, A = torch.randn(b, l, n, device=DEV), torch.randn(b, l, n, device=DEV), -torch.rand(d, n, device=DEV) - 0.1
+    D, bias = torch.randn(d, device=DEV), torch.randn(d, device=DEV)
+    got = []
+    for t in (u, u.contiguous()):
+        zz = z.clone().requires_grad_()
+        y = SS.selective_scan(t, dt, A, B, C, D, zz, bias)
+        got.append((y, *torch.autograd.grad(y, zz, g)))
+    for a, c in zip(*got):
+        assert torch.equal(a, c)
