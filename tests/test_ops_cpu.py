@@ -273,6 +273,6 @@ def test_scan_results_have_contiguous_channels(shape, stride):
     """The scan kernels write the last dimension with unit stride, also for an input of overlapping windows, whose dense copy
     puts time innermost."""
     from gpt_neox_b200.ops.selective_scan import _like_rows
-    new = _like_rows(torch.zeros(200).as_strided(shape, stride))
+    new = _like_rows(torch.zeros(400).as_strided(shape, stride))
     assert new.shape == shape and (new.stride(2) == 1 or shape[2] == 1)
     assert new.is_contiguous() or new.transpose(0, 1).is_contiguous()
