@@ -135,8 +135,10 @@ class GraphDecoder:
     numerics are tested.  The reference decodes with ``torch.cat`` caches and eager launches
     (``megatron/text_generation_utils.py:198-405``)."""
 
+    capacity = None             # rows of a cache
+
     def __init__(self, neox_args, model, batch_size, capacity, capture=None):
-        self.model = model
+        self.model, self.capacity = model, capacity
         dev = _dev()
         self.attn = [m for m in model.module.modules() if hasattr(m, "static_kv") and hasattr(m, "static_cache_supported")]
         self.supported = bool(self.attn) and all(m.static_cache_supported() and m.use_cache for m in self.attn)
@@ -183,6 +185,9 @@ class GraphDecoder:
 
     def step(self, tokens, position_ids, index):
         """Logits ``[b, 1, V]`` for the token at sequence position ``index`` given everything before it."""
+        # the step reads the position on the device, where one past the end can only be clamped (onto the last cached row)
+        if self.capacity is not None and not 0 <= int(index) < self.capacity:
+            raise IndexError(f"decoding step at position {int(index)} of a cache of {self.capacity} rows")
         self.tokens.copy_(tokens)
         self.position_ids.copy_(position_ids)
         self.pos.fill_(index)

@@ -425,3 +425,27 @@ def test_deepy_train_then_generate_from_the_checkpoint(tmp_path):
     assert (tmp_path / "ckpt" / "latest").read_text().strip() == "global_step4"
     samples = [json.loads(l) for l in open(tmp_path / "samples.txt")]
     assert len(samples) == 3 and all(s["length"] > 0 for s in samples)
+
+
+def test_decoding_step_outside_the_cache_is_refused():
+    """A fixed-capacity decoder refuses a position that its cache has no row for, before it touches anything."""
+    import torch
+    from gpt_neox_b200.text_generation import GraphDecoder
+
+    class Module(torch.nn.Module):
+        def forward(self, args):
+            return args[0].float()
+
+    class Model:
+        module = Module()
+
+    class Args:
+        params_dtype = torch.float32
+    d = GraphDecoder(Args, Model(), 2, 5, capture=False)
+    zeros = torch.zeros(2, 1, dtype=torch.long, device=d.tokens.device)
+    for index in (0, 4):
+        assert d.step(zeros + 7, zeros, index).tolist() == [[7.0]] * 2 and int(d.pos) == index
+    for index in (5, 6, -1):
+        with pytest.raises(IndexError):
+            d.step(zeros, zeros, index)
+    assert int(d.pos) == 4 and d.steps == 2
