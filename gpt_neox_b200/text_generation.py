@@ -13,6 +13,7 @@ from __future__ import annotations
 import copy
 import gc
 import json
+import threading
 import time
 from typing import List, Union
 
@@ -124,6 +125,30 @@ def stop_tokens_in_completion(stop_tokens, context_tokens, batch_index, current_
     return False
 
 
+class _collector_rests:
+    """No automatic garbage collection until the last of the threads inside has left; then it is as the first one found it.
+    (The switch is the interpreter's: were each thread to save and restore it by itself, the first to leave would turn the
+    collector on under the others.)"""
+
+    _lock, _inside, _was_on = threading.Lock(), 0, False
+
+    def __enter__(self):
+        cls = _collector_rests
+        with cls._lock:
+            if cls._inside == 0:
+                cls._was_on = gc.isenabled()
+                gc.disable()
+            cls._inside += 1
+
+    def __exit__(self, *exc):
+        cls = _collector_rests
+        with cls._lock:
+            cls._inside -= 1
+            if cls._inside == 0 and cls._was_on:
+                gc.enable()
+        return False
+
+
 class GraphDecoder:
     """Token-by-token decoding with a fixed-capacity key/value cache, replayed from a CUDA graph.
 
@@ -205,16 +230,11 @@ class GraphDecoder:
             torch.cuda.current_stream().wait_stream(side)
             # A model and its decoders refer to each other, so a decoder of a model that is gone waits for the garbage
             # collector; were its graph destroyed while this one is captured, the capture would be lost.
-            collecting = gc.isenabled()
-            gc.disable()
-            try:
+            with _collector_rests():
                 graph = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(graph):
                     self.logits = self._forward()
                 self.graph = graph
-            finally:
-                if collecting:
-                    gc.enable()
         self.graph.replay()
         return self.logits
 

@@ -449,3 +449,41 @@ def test_decoding_step_outside_the_cache_is_refused():
         with pytest.raises(IndexError):
             d.step(zeros, zeros, index)
     assert int(d.pos) == 4 and d.steps == 2
+
+
+@pytest.mark.parametrize("on", [True, False])
+def test_collector_rests_until_the_last_capture_ends(on):
+    """Captures of two threads that overlap: the one that ends first does not turn the collector on inside the other, and
+    afterwards it is as it was, also when a capture fails."""
+    import gc
+    import threading
+    from gpt_neox_b200.text_generation import _collector_rests
+    first_in, second_in, first_out, seen = threading.Event(), threading.Event(), threading.Event(), []
+
+    def first():
+        try:
+            with _collector_rests():
+                first_in.set()
+                second_in.wait(20)
+                seen.append(gc.isenabled())
+                raise RuntimeError("capture failed")
+        except RuntimeError:
+            first_out.set()
+
+    def second():
+        first_in.wait(20)
+        with _collector_rests():
+            second_in.set()
+            first_out.wait(20)
+            seen.append(gc.isenabled())
+    was = gc.isenabled()
+    (gc.enable if on else gc.disable)()
+    try:
+        threads = [threading.Thread(target=f) for f in (first, second)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(60)
+        assert seen == [False, False] and gc.isenabled() == on
+    finally:
+        (gc.enable if was else gc.disable)()
