@@ -249,3 +249,57 @@ def _expert_tensor_parallel(rank, world):
 
 def test_moe_expert_tensor_parallelism_matches_dense_math():
     run_distributed(_expert_tensor_parallel, 2)
+
+
+def _layer_epilogues(rank, world, cfg):
+    import torch
+    from common import make_args
+    from gpt_neox_b200.initialize import initialize_megatron
+    from gpt_neox_b200.models.init_functions import get_init_methods
+    from gpt_neox_b200.models.transformer import ParallelTransformerLayer
+    args = make_args(**{**cfg, "global_num_gpus": world, "model_parallel_size": world})
+    args.configure_distributed_args()
+    initialize_megatron(args)
+    init, out_init = get_init_methods(args)
+    layer = ParallelTransformerLayer(args, None, init, out_init, 0, rotary=True).float()
+    for name, p in layer.named_parameters():
+        if name.endswith("bias"):
+            torch.nn.init.normal_(p, std=0.5)
+    torch.manual_seed(1)
+    x0, g = torch.randn(12, 2, args.hidden_size), torch.randn(12, 2, args.hidden_size)
+
+    def plain(x):
+        """The block in separate operations: projections without residual, biases added by hand."""
+        add = lambda pair: pair[0] if pair[1] is None else pair[0] + pair[1]
+        if args.gpt_j_residual:
+            both = add(layer.attention(layer.input_layernorm(x))) + add(layer.mlp(layer.post_attention_layernorm(x)))
+            return x + (layer._reduce(both) if world > 1 else both)
+        x = x + add(layer.attention(layer.input_layernorm(x)))
+        return x + add(layer.mlp(layer.post_attention_layernorm(x)))
+    results = []
+    for run in (lambda x: layer(x)[0], plain):
+        layer.zero_grad()
+        x = x0.clone().requires_grad_()
+        y = run(x)
+        y.backward(g)
+        results.append([y.detach(), x.grad] + [p.grad.clone() for p in layer.parameters()])
+    for a, b in zip(*results):
+        torch.testing.assert_close(a, b, atol=2e-5, rtol=1e-4)
+    # a prompt and single tokens against the cache, in evaluation, where dropout is off whatever its probability
+    layer.hidden_dropout = 0.1
+    layer.eval()
+    want = results[1][0]
+    layer.use_cache = layer.attention.use_cache = True
+    with torch.no_grad():
+        parts = [layer(x0[:9])[0]] + [layer(x0[i:i + 1])[0] for i in range(9, 12)]
+    torch.testing.assert_close(torch.cat(parts), want, atol=2e-5, rtol=1e-4)
+
+
+@pytest.mark.parametrize("world,cfg", [
+    (1, {"gpt_j_residual": False}), (1, {"gpt_j_residual": True}),
+    (1, {"gpt_j_residual": False, "norm": "rmsnorm", "activation": "swiglu", "use_bias_in_mlp": False, "num_kv_heads": 2}),
+    (2, {"gpt_j_residual": False}), (2, {"gpt_j_residual": True})])
+def test_layer_with_biases_and_residual_in_its_projections(world, cfg):
+    """Biases and residuals that ride in the output projections give the block's sum of separate operations: training with all
+    gradients, and decoding against the cache, for both residual forms, with and without a reduction over ranks."""
+    run_distributed(_layer_epilogues, world, cfg)
