@@ -48,8 +48,8 @@ struct GemmParams {
     const int4* groups = nullptr;
     const int* group_ntiles = nullptr;
     int group_mode = 0;
-    // contraction split (plain tiles that accumulate in place into an fp32 output): every output tile is computed as
-    // `splits` partial tiles over consecutive runs of contraction blocks, which meet in the output's atomic additions
+    // contraction split (plain tiles, fp32 output): every output tile is computed as `splits` partial tiles over consecutive
+    // runs of contraction blocks; D is [splits * M, N], part by part
     int splits = 1;
 };
 
@@ -78,16 +78,16 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int tile, int num_m, int num_n, int nk_all) {
     TileInfo t;
     if (p.group_mode == 0) {
-        int m_blk, n_blk, k0 = 0, k1 = nk_all;
+        int m_blk, n_blk, part = 0, k0 = 0, k1 = nk_all;
         if (p.splits > 1) {
-            const int part = tile / (num_m * num_n);
+            part = tile / (num_m * num_n);
             tile -= part * num_m * num_n;
             k0 = (int)((long long)nk_all * part / p.splits);
             k1 = (int)((long long)nk_all * (part + 1) / p.splits);
         }
         tile_coords(tile, num_m, num_n, m_blk, n_blk);
         t.a_m0 = m_blk * BM; t.a_k0 = k0 * BK; t.b_n0 = n_blk * BN; t.b_k0 = k0 * BK; t.n0 = n_blk * BN; t.nk = k1 - k0;
-        t.row0 = m_blk * BM; t.row_end = p.M;
+        t.row0 = part * p.M + m_blk * BM; t.row_end = part * p.M + p.M;
     } else if (p.group_mode == 1) {
         const int4 g = __ldg(p.groups + tile);
         t.a_m0 = g.x; t.a_k0 = 0; t.n0 = g.w * BN; t.nk = nk_all;
@@ -216,10 +216,6 @@ __device__ __forceinline__ void epilogue_chunk_t(const uint32_t (&r)[32], int ro
             if (p.preact) st_16<H16>(p.preact, (long long)row * p.ldpre + col, x);
             if (p.act == 1) x = gelu_tanh(x);
             else if (p.act == 2) x *= dgelu_tanh(ld_16<H16>(p.aux, (long long)row * p.ldaux + col));
-            if (p.splits > 1) {
-                atomicAdd(reinterpret_cast<float*>(p.D) + (long long)row * p.ldd + col, x);
-                continue;
-            }
             if (p.add) {
                 if (p.add_fp32) x += reinterpret_cast<const float*>(p.add)[(long long)row * p.ldadd + col];
                 else x += ld_16<H16>(p.add, (long long)row * p.ldadd + col);

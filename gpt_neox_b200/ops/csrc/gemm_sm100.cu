@@ -17,6 +17,7 @@
 // All barrier waits are bounded (see sm100_ptx.cuh); on a time-out the kernel records a code in the
 // status word, leaves its loops, frees its tensor memory and returns.
 #include "gemm_common.cuh"
+#include "launch.cuh"
 #include "neox_b200.h"
 #include <mutex>
 #include <unordered_map>
@@ -66,6 +67,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+
+    if (p.splits > 1) launch::let_successor_start();        // add_parts_kernel, which waits for this one
 
     const int num_m = (p.M + BM - 1) / BM;
     const int num_n = (p.N + BN - 1) / BN;
@@ -350,23 +353,67 @@ extern "C" int neox_gemm_bf16_rowmap(const void* A, const void* B, void* D, int 
                         aux, ldaux, act, alpha, row_ptrs, 0, stream_);
 }
 
-// Contraction splits of an accumulating product.  Weight gradients of narrow models have few output tiles and a long
-// contraction (all tokens): 768 x 768 over 8192 tokens is 18 tiles, each walking 128 k-blocks while 130 SMs idle.  The
-// cost of a choice is rounds of tiles x blocks per tile; splits are taken while they cut that by an eighth and leave a
-// tile 8 k-blocks, below which filling the pipeline and the epilogue's atomic pass over the tile outweigh the product.
-// Mean over a 125M model's four weight gradients (8192 tokens) 56.6 -> 35.4 us, a Mamba-130M's 41.9 -> 24.9 us.  The order
-// of the additions to an element is not fixed.
-static int pick_splits(long long tiles, int nk, int sms) {
-    int best = 1;
-    double cost = (double)((tiles + sms - 1) / sms) * nk;
-    for (int s = 2; s <= 8 && nk / s >= 8; ++s) {
-        const double c = (double)((tiles * s + sms - 1) / sms) * ((nk + s - 1) / s);
-        if (c < cost * 0.875) {
-            best = s;
-            cost = c;
+constexpr int MAX_SPLITS = 8;
+
+// D[m][n] += parts[0][m][n] + parts[1][m][n] + ..., always in this order.  parts: [splits][M][pitch].  Bound by its bytes, which
+// the product has just left in L2, and by its launch: its blocks are let in while the product runs and wait for its end, all
+// parts of an element are requested at once (768 x 768, 8 parts: about 5 us with the writing of the parts, 7 without either).
+template <int VEC>
+static __global__ void __launch_bounds__(256)
+add_parts_kernel(float* D, long long ldd, const float* parts, int M, int N, int pitch, int splits) {
+    struct alignas(VEC * 4) Pack {
+        float v[VEC];
+    };
+    launch::wait_for_predecessor();
+    const int nv = N / VEC;
+    const long long i = blockIdx.x * 256ll + threadIdx.x, stride = (long long)M * pitch;
+    if (i >= (long long)M * nv) return;
+    const int row = (int)(i / nv), col = (int)(i - (long long)row * nv) * VEC;
+    const float* src = parts + (long long)row * pitch + col;
+    Pack p[MAX_SPLITS];
+#pragma unroll
+    for (int s = 0; s < MAX_SPLITS; ++s)
+        if (s < splits) p[s] = *reinterpret_cast<const Pack*>(src + s * stride);
+    Pack* dst = reinterpret_cast<Pack*>(D + (long long)row * ldd + col);
+    Pack d = *dst;
+#pragma unroll
+    for (int s = 1; s < MAX_SPLITS; ++s) {
+        if (s < splits) {
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) p[0].v[j] += p[s].v[j];
         }
     }
-    return best;
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) d.v[j] += p[0].v[j];
+    *dst = d;
+}
+
+// Operands, tensor maps and launch of everything that runs on gemm_bf16_tcgen05_kernel without a tile table; p holds the rest.
+static int launch_tiles(const void* A, const void* B, long long lda, long long ldb, GemmParams& p, cudaStream_t stream) {
+    // TMA constraints: 16-byte aligned base, row pitch a multiple of 16 bytes.
+    if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda % 8) || (ldb % 8))
+        return NEOX_ERR_ALIGN;
+    p.status = neox_status_word();
+    if (!p.status) return NEOX_ERR_DRIVER;
+    CUtensorMap tmA, tmB;
+    int rc;
+    if (!p.a_mn) rc = neox_make_tmap_bf16_2d(&tmA, A, p.K, p.M, lda, BK, BM);
+    else rc = neox_make_tmap_bf16_2d(&tmA, A, p.M, p.K, lda, 64, BK);
+    if (rc) return rc;
+    if (!p.b_mn) rc = neox_make_tmap_bf16_2d(&tmB, B, p.K, p.N, ldb, BK, BN);
+    else rc = neox_make_tmap_bf16_2d(&tmB, B, p.N, p.K, ldb, 64, BK);
+    if (rc) return rc;
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             SMEM_BYTES);
+        if (e != cudaSuccess) return NEOX_ERR_LAUNCH;
+        attr_set = true;
+    }
+    const int num_m = (p.M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
+    const long long tiles = (long long)num_m * num_n * p.splits, sms = neox_sm_count();
+    gemm_bf16_tcgen05_kernel<<<(int)(tiles < sms ? tiles : sms), NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+    return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
 // The general entry point: h16 = 0 for bf16, 1 for fp16 (operands and every 16-bit epilogue tensor share the type).
@@ -374,24 +421,8 @@ extern "C" int neox_gemm_16(const void* A, const void* B, void* D, int M, int N,
                             long long ldd, int a_mn, int b_mn, int d_fp32, const void* bias, const void* add,
                             long long ldadd, int add_fp32, void* preact, long long ldpre, const void* aux,
                             long long ldaux, int act, float alpha, const void* row_ptrs, int h16, void* stream_) {
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (row_ptrs && d_fp32) return NEOX_ERR_SHAPE;
     if (M <= 0 || N <= 0 || K <= 0) return 0;
-    // TMA constraints: 16-byte aligned base, row pitch a multiple of 16 bytes.
-    if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda % 8) || (ldb % 8))
-        return NEOX_ERR_ALIGN;
-    int* status = neox_status_word();
-    if (!status) return NEOX_ERR_DRIVER;
-
-    CUtensorMap tmA, tmB;
-    int rc;
-    if (!a_mn) rc = neox_make_tmap_bf16_2d(&tmA, A, K, M, lda, BK, BM);
-    else rc = neox_make_tmap_bf16_2d(&tmA, A, M, K, lda, 64, BK);
-    if (rc) return rc;
-    if (!b_mn) rc = neox_make_tmap_bf16_2d(&tmB, B, K, N, ldb, BK, BN);
-    else rc = neox_make_tmap_bf16_2d(&tmB, B, N, K, ldb, 64, BK);
-    if (rc) return rc;
-
     GemmParams p;
     p.M = M; p.N = N; p.K = K;
     p.a_mn = a_mn; p.b_mn = b_mn;
@@ -401,7 +432,6 @@ extern "C" int neox_gemm_16(const void* A, const void* B, void* D, int M, int N,
     p.preact = static_cast<__nv_bfloat16*>(preact); p.ldpre = ldpre;
     p.aux = static_cast<const __nv_bfloat16*>(aux); p.ldaux = ldaux;
     p.act = act; p.alpha = alpha;
-    p.status = status;
     p.row_ptrs = static_cast<const unsigned long long*>(row_ptrs);
     p.h16 = h16 ? 1 : 0;
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
@@ -411,22 +441,58 @@ extern "C" int neox_gemm_16(const void* A, const void* B, void* D, int M, int N,
     if (preact) vec = vec && al16(preact) && (ldpre % 8 == 0);
     if (aux) vec = vec && al16(aux) && (ldaux % 8 == 0);
     p.vec_ok = vec ? 1 : 0;
+    return launch_tiles(A, B, lda, ldb, p, static_cast<cudaStream_t>(stream_));
+}
 
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             SMEM_BYTES);
-        if (e != cudaSuccess) return NEOX_ERR_LAUNCH;
-        attr_set = true;
+// Contraction splits of an accumulating product (1: use neox_gemm_16).  Weight gradients of narrow models have few output
+// tiles and a long contraction (all tokens): 768 x 768 over 8192 tokens is 18 tiles, each walking 128 k-blocks while 130 SMs
+// idle.  Every tile is computed in `splits` parts, written to a workspace, and a second pass adds the parts to the output one
+// after the other, so the result is bitwise repeatable.  (Parts that meet in atomic additions are faster, as they need neither
+// workspace nor pass, but their order is not fixed.)  The cost of a choice, in k-blocks of 0.43 us, is rounds of tiles x blocks
+// per tile, and for a split the launch of the second pass (8) and the bytes of workspace and output (2.5 per million elements
+// and pass over them).  Fitted to 2 to 8 parts of 21 shapes over 512 to 16384 rows; on average 0.2 % off the best of them.
+// us over 8192 rows, whole / split / with atomics: 768 x 768 59 / 26 / 21, 2304 x 768 61 / 47 / 42, 3072 x 768 63 / 50 / 42,
+// 1024 x 1024 59 / 29 / 26, 80 x 1536 57 / 20 / 16; over 2048 rows 768 x 768 23 / 21 / 15, 3072 x 768 24, left whole / 21.
+extern "C" int neox_gemm_splits(int M, int N, int K) {
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN), sms = neox_sm_count();
+    const int nk = (K + BK - 1) / BK;
+    int best = 1;
+    double cost = (double)((tiles + sms - 1) / sms) * nk;
+    for (int s = 2; s <= MAX_SPLITS && nk / s >= 4; ++s) {
+        const double c = (double)((tiles * s + sms - 1) / sms) * ((nk + s - 1) / s) + 8.0 + 2.5e-6 * (s + 1.0) * M * N;
+        if (c < cost) {
+            best = s;
+            cost = c;
+        }
     }
-    const int num_m = (M + BM - 1) / BM, num_n = (N + BN - 1) / BN;
-    const int sms = neox_sm_count();
-    const bool inplace = d_fp32 && add_fp32 && add == D && ldadd == ldd && !preact && act == 0 && !bias;
-    if (inplace) p.splits = pick_splits((long long)num_m * num_n, (K + BK - 1) / BK, sms);
-    long long grid = (long long)num_m * num_n * p.splits;
-    if (grid > sms) grid = sms;
-    gemm_bf16_tcgen05_kernel<<<(int)grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
-    return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
+    return best;
+}
+
+// D (fp32) += alpha * op(A) op(B) in `splits` parts; parts: splits * M * (N rounded up to 4) floats of workspace.
+extern "C" int neox_gemm_accumulate_16(const void* A, const void* B, float* D, int M, int N, int K, long long lda, long long ldb,
+                                       long long ldd, int a_mn, int b_mn, float alpha, int splits, float* parts, int h16,
+                                       void* stream_) {
+    if (M <= 0 || N <= 0 || K <= 0) return 0;
+    const long long pitch = (N + 3) / 4 * 4ll;
+    if (splits < 1 || splits > MAX_SPLITS || splits > (K + BK - 1) / BK || (long long)splits * M > 0x7fffffff) return NEOX_ERR_SHAPE;
+    if (reinterpret_cast<uintptr_t>(parts) & 15) return NEOX_ERR_ALIGN;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    GemmParams p;
+    p.M = M; p.N = N; p.K = K;
+    p.a_mn = a_mn; p.b_mn = b_mn;
+    p.D = parts; p.ldd = pitch; p.d_fp32 = 1;
+    p.bias = nullptr; p.add = nullptr; p.ldadd = 0; p.add_fp32 = 0;
+    p.preact = nullptr; p.ldpre = 0; p.aux = nullptr; p.ldaux = 0;
+    p.act = 0; p.alpha = alpha; p.vec_ok = 1; p.row_ptrs = nullptr;
+    p.h16 = h16 ? 1 : 0;
+    p.splits = splits;
+    const int rc = launch_tiles(A, B, lda, ldb, p, stream);
+    if (rc) return rc;
+    const bool vec = N % 4 == 0 && ldd % 4 == 0 && !(reinterpret_cast<uintptr_t>(D) & 15);
+    const long long items = (long long)M * (vec ? N / 4 : N), blocks = (items + 255) / 256;
+    if (blocks > 0x7fffffff) return NEOX_ERR_SHAPE;
+    return launch::overlapped(vec ? add_parts_kernel<4> : add_parts_kernel<1>, dim3((int)blocks), dim3(256), 1, stream, D, ldd,
+                              parts, M, N, (int)pitch, splits);
 }
 
 // ------------------------------------------------------------------------------------------------------------

@@ -106,6 +106,12 @@ def gemm_rowmap(a, b, row_ptrs, b_mn=False, bias=None):
     native.check(rc, "neox_gemm_bf16_rowmap")
 
 
+def _accumulates(out, bias, add, act, pre):
+    """``out += alpha * op(a) @ op(b)`` in fp32 and nothing else: the form that may split its contraction."""
+    return (add is not None and out.dtype == torch.float32 and add.dtype == torch.float32 and bias is None
+            and act == ACT_NONE and pre is None and add.data_ptr() == out.data_ptr() and add.stride(0) == out.stride(0))
+
+
 def gemm(a, b, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, bias=None, add=None, act=ACT_NONE,
          aux=None, alpha=1.0, want_preact=False):
     """See module docstring.  ``add`` may alias ``out`` (in-place accumulate, e.g. wgrad into main_grad)."""
@@ -155,7 +161,13 @@ def gemm(a, b, a_mn=False, b_mn=False, out=None, out_dtype=torch.bfloat16, bias=
     elif use_pair_kernel(M, N, K):
         rc = L.neox_gemm_16_2cta(*head, int(a_mn), int(b_mn), *epilogue, h16, native.stream_ptr())
     else:
-        rc = L.neox_gemm_16(*head, int(a_mn), int(b_mn), *epilogue, None, h16, native.stream_ptr())
+        splits = L.neox_gemm_splits(M, N, K) if _accumulates(out, bias, add, act, pre) else 1
+        if splits > 1:
+            parts = torch.empty(splits * M * ((N + 3) // 4 * 4), dtype=torch.float32, device=a.device)
+            rc = L.neox_gemm_accumulate_16(*head, int(a_mn), int(b_mn), alpha, splits, parts.data_ptr(), h16,
+                                           native.stream_ptr())
+        else:
+            rc = L.neox_gemm_16(*head, int(a_mn), int(b_mn), *epilogue, None, h16, native.stream_ptr())
     if rc:
         native.check(rc, "neox_gemm_16")
     return (out, pre) if want_preact else out

@@ -43,6 +43,8 @@ _GEMM_EPILOGUE = [c_int, c_void_p, c_void_p, c_ll, c_int, c_void_p, c_ll, c_void
 _ARGTYPES = {
     "neox_gemm_skinny_16": [*_GEMM_HEAD, *_GEMM_EPILOGUE, c_int, c_void_p],
     "neox_gemm_16": [*_GEMM_HEAD, c_int, c_int, *_GEMM_EPILOGUE, c_void_p, c_int, c_void_p],
+    "neox_gemm_splits": [c_int, c_int, c_int],
+    "neox_gemm_accumulate_16": [*_GEMM_HEAD, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p],
     "neox_gemm_16_2cta": [*_GEMM_HEAD, c_int, c_int, *_GEMM_EPILOGUE, c_int, c_void_p],
 }
 
@@ -52,7 +54,8 @@ launch_count = 0   # number of kernel-launching library calls made by this proce
 class _CountingLib:
     """Proxy over the CDLL that counts calls into kernel launchers (``neox_*`` entry points that take a
     stream); pure queries such as ``neox_read_status`` are not counted."""
-    _NOT_LAUNCHES = {"neox_read_status", "neox_norm_bwd_blocks", "neox_sm_count_c", "neox_causal_conv_blocks"}
+    _NOT_LAUNCHES = {"neox_read_status", "neox_norm_bwd_blocks", "neox_sm_count_c", "neox_causal_conv_blocks",
+                     "neox_gemm_splits"}
 
     def __init__(self, cdll):
         self._cdll = cdll

@@ -1336,3 +1336,31 @@ def test_selective_scan_on_overlapping_windows():
         got.append((y, *torch.autograd.grad(y, zz, g)))
     for a, c in zip(*got):
         assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(128, 256, 8192), (136, 40, 4104), (768, 768, 1000), (72, 1030, 3000), (200, 264, 700),
+                                   (768, 2304, 8192)])
+def test_accumulating_gemm_is_repeatable(M, N, K, dtype):
+    """``acc += a^T b`` gives the same bits every time, whatever order the parts of a split contraction finish in, and touches
+    nothing beside the product's columns when the output is a slice of a wider buffer.  Values: the tensor cores truncate the
+    running sum (about 5 sqrt(K) at most for products of unit normals) to 24 bits after each of K / 16 steps."""
+    torch.manual_seed(K)
+    a, b = torch.randn(K, M, device=DEV).to(dtype), torch.randn(K, (N + 7) // 8 * 8, device=DEV).to(dtype)[:, :N]
+    wide = torch.randn(M, N + 3, device=DEV)
+    results = []
+    for view in (lambda t: t[:, :N], lambda t: t[:, 3:]):
+        for _ in range(6):
+            acc = wide.clone()
+            G.gemm(a, b, a_mn=True, b_mn=True, out=view(acc), add=view(acc))
+            keep = acc.clone()
+            view(keep).copy_(view(wide))
+            assert torch.equal(keep, wide)
+            results.append(view(acc).clone())
+        want = view(wide).double() + a.double().t() @ b.double()
+        _close(results[-1], want, K / 16 * 2.0 ** -23 * 5 * math.sqrt(K), rtol=1e-5)
+        assert all(torch.equal(r, results[-1]) for r in results[-6:])
+    dense = [wide[:, :N].clone() for _ in range(6)]
+    for t in dense:
+        G.gemm(a, b, a_mn=True, b_mn=True, out=t, add=t)
+    assert all(torch.equal(t, results[0]) for t in dense)
