@@ -322,9 +322,10 @@ extern "C" int neox_wkv6_bwd(int B, int T, int C, int H, const void* r, const vo
                              const void* u, const void* gy, void* gr, void* gk, void* gv, void* gw, float* cum,
                              float* gu_part, void* stream) {
     if (C % H) return NEOX_ERR_SHAPE;
-    if (B <= 0 || T <= 0) return 0;
+    if (B <= 0) return 0;
     const int n = C / H;
     cudaStream_t st = (cudaStream_t)stream;
+    if (T <= 0) return cudaMemsetAsync(gu_part, 0, (size_t)B * C * sizeof(float), st) == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
     const Shape sh{T, C, H};
     float* cumB = cum + (size_t)B * T * C;
     WKV_DISPATCH(n, {

@@ -1364,3 +1364,18 @@ def test_accumulating_gemm_is_repeatable(M, N, K, dtype):
     for t in dense:
         G.gemm(a, b, a_mn=True, b_mn=True, out=t, add=t)
     assert all(torch.equal(t, results[0]) for t in dense)
+
+
+@pytest.mark.parametrize("B,H", [(1, 2), (3, 4)])
+def test_wkv6_without_steps_has_zero_gradients(B, H):
+    """No steps: empty results, and a gradient of zero for the bonus, whatever was in memory before."""
+    from gpt_neox_b200.ops import wkv6 as W
+    N = 64
+    r, k, v, w = (torch.zeros(B, 0, H * N, device=DEV, dtype=torch.bfloat16, requires_grad=True) for _ in range(4))
+    u = torch.randn(H, N, device=DEV).to(torch.bfloat16).requires_grad_()
+    y = W.wkv6(r, k, v, w, u)
+    assert y.shape == (B, 0, H * N)
+    for _ in range(4):
+        torch.full((B, H, N), float("nan"), device=DEV)                       # what a fresh allocation may hold
+        grads = torch.autograd.grad(y, (r, k, v, w, u), torch.empty_like(y), retain_graph=True)
+        assert all(g.numel() == 0 for g in grads[:4]) and torch.equal(grads[4], torch.zeros_like(u))
