@@ -100,6 +100,16 @@ scan_state_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const
     sumd[((size_t)b * nchk + ck) * d + c] = total;
 }
 
+// h * 2^x + add: the state that a chunk of decay 2^x hands on.  The decay of 32 steps may leave the range of fp32 although the
+// state, taken step by step, does not: then it is applied in two halves.  A state of 0 stays 0 and one that has overflowed stays
+// so.
+__device__ __forceinline__ float carry(float h, float x, float add) {
+    if (fabsf(x) < 126.f) return __fmaf_rn(exp2f(x), h, add);
+    if (h == 0.f || isinf(h)) return h + add;
+    const float half = exp2f(0.5f * x);
+    return __fmaf_rn(half * h, half, add);
+}
+
 // ------------------------------------------------------------------ combine over the chunks, in place
 // Forward: slot k + 1 holds the state that chunk k adds; afterwards the state at the start of chunk k + 1.
 // Reverse: slot k - 1 holds the adjoint that chunk k adds; afterwards the adjoint arriving at the end of chunk k - 1.
@@ -117,14 +127,14 @@ scan_combine_kernel(const float* __restrict__ A, const float* __restrict__ sumd,
             if (k0 + i < nchk - 1) {
                 const int k = REVERSE ? nchk - 1 - (k0 + i) : k0 + i;
                 loc[i] = st[slot(b, REVERSE ? k - 1 : k + 1, nchk, d) + (size_t)j * d + c];
-                dec[i] = exp2f(a * sumd[((size_t)b * nchk + k) * d + c]);
+                dec[i] = a * sumd[((size_t)b * nchk + k) * d + c];
             }
         }
 #pragma unroll
         for (int i = 0; i < GROUP; ++i) {
             if (k0 + i < nchk - 1) {
                 const int k = REVERSE ? nchk - 1 - (k0 + i) : k0 + i;
-                h = h == 0.f ? loc[i] : dec[i] * h + loc[i];      // nothing to carry: a decay of inf must not make NaN of 0
+                h = carry(h, dec[i], loc[i]);
                 st[slot(b, REVERSE ? k - 1 : k + 1, nchk, d) + (size_t)j * d + c] = h;
             }
         }

@@ -1379,3 +1379,27 @@ def test_wkv6_without_steps_has_zero_gradients(B, H):
         torch.full((B, H, N), float("nan"), device=DEV)                       # what a fresh allocation may hold
         grads = torch.autograd.grad(y, (r, k, v, w, u), torch.empty_like(y), retain_graph=True)
         assert all(g.numel() == 0 for g in grads[:4]) and torch.equal(grads[4], torch.zeros_like(u))
+
+
+@pytest.mark.parametrize("first", [1e30, float("inf"), -float("inf")])
+def test_selective_scan_carries_extreme_states_between_chunks(first):
+    """A state that is huge, or has overflowed, and decays by more than fp32's range over a chunk of 32 steps, though by a normal
+    number in each: it is handed on as in the step-by-step recurrence.  (Outputs in bf16, 2^-8 each; 96 factors of a relative
+    error of 2^-22 and an exponent of up to 400 in each product of factors.)"""
+    from gpt_neox_b200.ops import selective_scan as SS
+    b, l, d, n = 1, 100, 64, 16
+    u = torch.zeros(b, l, d, device=DEV).to(torch.bfloat16)
+    u[:, 0] = first
+    dt = torch.full((b, l, d), 0.5413, device=DEV).to(torch.bfloat16)          # softplus: 1
+    A = -torch.linspace(0.5, 4.0, d, device=DEV)[:, None].expand(d, n).contiguous()
+    B, C, z = torch.ones(b, l, n, device=DEV), torch.ones(b, l, n, device=DEV), torch.ones(b, l, d, device=DEV).to(torch.bfloat16)
+    D, bias = torch.zeros(d, device=DEV), torch.zeros(d, device=DEV)
+    got = SS.selective_scan(u, dt, A, B, C, D, z, bias).float()
+    want = SS.selective_scan_ref(u.double(), dt.double(), A.double(), B.double(), C.double(), D.double(), z.double(), bias.double(),
+                                 True) if math.isfinite(first) else None
+    if want is not None:
+        normal = want.abs() > 2.0 ** -120
+        assert int(normal[:, 64:].sum()) > 0
+        assert bool(((got.double() - want).abs() <= 0.01 * want.abs())[normal].all())
+    else:
+        assert bool((got[:, 1:] == first).all())
