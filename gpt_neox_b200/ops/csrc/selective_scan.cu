@@ -18,6 +18,7 @@
 // the latency of every step: 1987 us forward, 7232 us backward at b 4, l 2048, d 1536.  The chunked form computes the
 // exponentials twice and has 64 times the threads: 181 us forward (state 67, combine 10, output 104) and 514 us backward
 // (adjoint 82, combine 15, gradient 417).  Exponentials alone would take 45 us a pass.
+#include "dynamic_smem.h"
 #include "neox_b200.h"
 #include <cuda_bf16.h>
 
@@ -518,13 +519,7 @@ extern "C" int neox_selective_scan_bwd(const void* u, const void* dt, const floa
     if (n != NS) return NEOX_ERR_SHAPE;
     if (b <= 0 || l <= 0 || d <= 0) return 0;
     const int nchk = (l + CHUNK - 1) / CHUNK;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(scan_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem)) !=
-            cudaSuccess)
-            return NEOX_ERR_LAUNCH;
-        attr_set = true;
-    }
+    if (!allow_dynamic_smem<scan_grad_kernel>(sizeof(GradSmem))) return NEOX_ERR_LAUNCH;
     const Strides st = make_strides(strides, 10);
     cudaStream_t cs = static_cast<cudaStream_t>(stream);
     const int dblk = (d + THREADS - 1) / THREADS, gblk = (d + GCH - 1) / GCH;

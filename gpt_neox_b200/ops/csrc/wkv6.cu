@@ -28,6 +28,7 @@
 // faster still, 80 us forward, but a sum taken in another order changes the last bit of some of the 16-bit results, and
 // twelve layers turn that into differences of 2 % between two training steps.)  The three backward scans share one
 // launch, so they run side by side.  Now 108 us forward, 108 us for the three scans and 29 us for the decay gradient.
+#include "dynamic_smem.h"
 #include "neox_b200.h"
 #include <cuda_bf16.h>
 
@@ -285,12 +286,6 @@ __global__ void __launch_bounds__(64) wkv6_decay_kernel(int T, int C, long long 
     }
 }
 
-template <typename K>
-bool allow_smem(K kernel, size_t bytes) {
-    return bytes <= 48 * 1024 ||
-           cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
-}
-
 #define WKV_DISPATCH(N_, ...)                                       \
     switch (N_) {                                                   \
         case 32: { constexpr int N = 32; __VA_ARGS__; break; }             \
@@ -310,7 +305,7 @@ extern "C" int neox_wkv6_fwd(int B, int T, int C, int H, const void* r, const vo
     const Shape sh{T, C, H};
     WKV_DISPATCH(n, {
         const size_t bytes = sizeof(ValueSmem<N>);
-        if (!allow_smem(wkv6_fwd_kernel<N>, bytes)) return NEOX_ERR_LAUNCH;
+        if (!allow_dynamic_smem<wkv6_fwd_kernel<N>>(bytes)) return NEOX_ERR_LAUNCH;
         wkv6_fwd_kernel<N><<<B * H, N * SLICES, bytes, st>>>(sh, (const bf16*)r, (const bf16*)k, (const bf16*)v, ew,
                                                              (const bf16*)u, (bf16*)y);
     });
@@ -330,7 +325,7 @@ extern "C" int neox_wkv6_bwd(int B, int T, int C, int H, const void* r, const vo
     float* cumB = cum + (size_t)B * T * C;
     WKV_DISPATCH(n, {
         const size_t bytes = sizeof(KeySmem<N>) > sizeof(ValueSmem<N>) ? sizeof(KeySmem<N>) : sizeof(ValueSmem<N>);
-        if (!allow_smem(wkv6_bwd_kernel<N>, bytes)) return NEOX_ERR_LAUNCH;
+        if (!allow_dynamic_smem<wkv6_bwd_kernel<N>>(bytes)) return NEOX_ERR_LAUNCH;
         wkv6_bwd_kernel<N><<<dim3(B * H, 3), N * SLICES, bytes, st>>>(sh, (const bf16*)r, (const bf16*)k, (const bf16*)v, ew,
                                                                      (const bf16*)u, (const bf16*)gy, (bf16*)gr, (bf16*)gk,
                                                                      (bf16*)gv, cum, cumB, gu_part);

@@ -276,3 +276,48 @@ def test_scan_results_have_contiguous_channels(shape, stride):
     new = _like_rows(torch.zeros(400).as_strided(shape, stride))
     assert new.shape == shape and (new.stride(2) == 1 or shape[2] == 1)
     assert new.is_contiguous() or new.transpose(0, 1).is_contiguous()
+
+
+def _run_cpp(tmp_path, source, cuda_headers=False):
+    """Compile ``source`` against the kernels' headers with the host compiler alone and run it; returns what it prints."""
+    import shutil
+    import subprocess
+    from pathlib import Path
+    import gpt_neox_b200.ops
+    include = ["-I", str(Path(gpt_neox_b200.ops.__file__).parent / "csrc")]
+    if cuda_headers:
+        home = Path("/usr/local/cuda/include")
+        if not (home / "cuda_runtime.h").exists():
+            pytest.skip("no CUDA headers")
+        include += ["-I", str(home)]
+    if shutil.which("g++") is None:
+        pytest.skip("no C++ compiler")
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text(source)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", *include, str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+
+
+def test_dynamic_shared_memory_is_allowed_on_every_device(tmp_path):
+    """The permission for large dynamic shared memory belongs to a device: asked for once per kernel and device, again after a
+    failure, and on every device a process uses.  The runtime calls are stand-ins."""
+    out = _run_cpp(tmp_path, r"""
+#include "dynamic_smem.h"
+#include <cstdio>
+static int dev = 0, calls = 0;
+static cudaError_t answer = cudaSuccess;
+extern "C" cudaError_t cudaGetDevice(int* d) { *d = dev; return cudaSuccess; }
+extern "C" cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { ++calls; return answer; }
+static void first(int) {}
+static void second(int) {}
+int main() {
+    auto show = [](bool ok) { std::printf("%d/%d ", (int)ok, calls); };
+    answer = cudaErrorInvalidValue; show(allow_dynamic_smem<first>(70000));
+    answer = cudaSuccess;
+    show(allow_dynamic_smem<first>(70000)); show(allow_dynamic_smem<first>(70000));
+    show(allow_dynamic_smem<second>(70000));
+    dev = 1; show(allow_dynamic_smem<first>(70000)); show(allow_dynamic_smem<first>(70000));
+    dev = 70; show(allow_dynamic_smem<first>(70000)); show(allow_dynamic_smem<first>(70000));
+    dev = 0; show(allow_dynamic_smem<first>(70000));
+}""", cuda_headers=True)
+    assert out.split() == ["0/1", "1/2", "1/2", "1/3", "1/4", "1/4", "1/5", "1/6", "1/6"]
