@@ -472,10 +472,10 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
 }
 
 // Chunks side by side, or all chunks of a channel in one block?  Side by side costs the exponentials twice, so it is
-// left where the channels alone fill the machine: 8 blocks of 128 on each of 148 SMs.
+// left where the channels alone fill the machine: 8 blocks of 128 on every SM.
 int forward_span(int b, int d, int nchk) {
     const long long blocks = (long long)b * ((d + THREADS - 1) / THREADS);
-    return nchk == 1 || blocks >= 148 * 8 ? nchk : 1;
+    return nchk == 1 || blocks >= 8ll * neox_sm_count() ? nchk : 1;
 }
 
 Strides make_strides(const long long* s, int operands) {
