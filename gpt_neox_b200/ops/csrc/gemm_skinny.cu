@@ -42,9 +42,10 @@ struct SkinnyParams {
     GemmParams e;                 // shape and epilogue
 };
 
-__device__ __forceinline__ uint4 load_stream(const void* p) {        // W: used once
+// W: used once.  A coherent load, as for X: the second operand of a product may be what the kernel in front has just written.
+__device__ __forceinline__ uint4 load_stream(const void* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;

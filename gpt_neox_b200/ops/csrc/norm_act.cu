@@ -171,8 +171,9 @@ __device__ __forceinline__ float row_sum(float v, float (&red)[32]) {
 
 template <typename T, bool RMS, int V, bool WARP>
 __global__ void __launch_bounds__(WARP ? ROW_WARPS * 32 : CTA_THREADS)
-norm_fwd_kernel(const T* x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
-                float* __restrict__ stat0, float* __restrict__ stat1, int rows, int cols, float eps) {
+norm_fwd_kernel(const T* x, const T* gamma, const T* beta, T* y, float* __restrict__ stat0, float* __restrict__ stat1,
+                int rows, int cols, float eps) {
+    // (no __restrict__ on x, gamma and beta: the compiler would read them as constants of the kernel's life, see launch.cuh)
     __shared__ float red0[32], red1[32];
     constexpr bool CACHED = V > 0;
     const int nvec = cols >> 3;

@@ -321,3 +321,22 @@ int main() {
     dev = 0; show(allow_dynamic_smem<first>(70000));
 }""", cuda_headers=True)
     assert out.split() == ["0/1", "1/2", "1/2", "1/3", "1/4", "1/4", "1/5", "1/6", "1/6"]
+
+
+def test_kernels_that_start_early_use_no_read_only_loads():
+    """A kernel that waits for the launch in front lives through that one's writes, so none of its loads may assume constant data:
+    no read-only load instruction, and no ``const __restrict__`` parameter, of which the compiler makes such loads."""
+    import re
+    from pathlib import Path
+    import gpt_neox_b200.ops
+    seen = 0
+    for path in sorted((Path(gpt_neox_b200.ops.__file__).parent / "csrc").glob("*.cu")):
+        text = path.read_text()
+        kernels = [k for k in re.split(r"(?=\n(?:static )?__global__ )", text)[1:] if "wait_for_predecessor()" in k.split("\n}\n")[0]]
+        for k in kernels:
+            body = k.split("\n}\n")[0]
+            assert not re.search(r"const\s+\w+\s*\*\s*__restrict__|__ldg\(", body), (path.name, body[:200])
+        if kernels:
+            assert "ld.global.nc" not in text, path.name
+        seen += len(kernels)
+    assert seen >= 4

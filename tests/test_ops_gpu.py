@@ -1403,3 +1403,31 @@ def test_selective_scan_carries_extreme_states_between_chunks(first):
         assert bool(((got.double() - want).abs() <= 0.01 * want.abs())[normal].all())
     else:
         assert bool((got[:, 1:] == first).all())
+
+
+def test_overlapped_kernels_read_what_the_launch_before_wrote():
+    """A product whose second operand, and norms whose scale and bias, are results of the overlapped launch right before, many
+    times over in recycled memory: the values of the same calls with a wait in between."""
+    torch.manual_seed(0)
+    cols, n = 1024, 256
+    src = [torch.randn(n, cols, device=DEV).to(torch.bfloat16) for _ in range(40)]
+    x, ones, zeros = (t.to(torch.bfloat16) for t in (torch.randn(3, cols, device=DEV), torch.ones(cols, device=DEV), torch.zeros(cols, device=DEV)))
+
+    def step(s, wait):
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        w = OF.layer_norm(s, ones, zeros, 1e-5)
+        sync()
+        y = G.gemm(x, w)                                       # [3, n]
+        sync()
+        scale, bias = (G.gemm(s[i:i + 1, :], s) for i in (0, 1))         # [1, n] each
+        sync()
+        a = OF.layer_norm(y, scale.view(-1), bias.view(-1), 1e-5)
+        b = OF.rms_norm(y, G.gemm(s[2:3, :], s).view(-1), None, 1e-5)
+        return y, a, b
+    with torch.no_grad():
+        want = [step(s, True) for s in src]
+        torch.cuda.synchronize()
+        for _ in range(5):
+            got = [step(s, False) for s in src]
+            for p, q in zip(want, got):
+                assert all(torch.equal(s, t) for s, t in zip(p, q))
