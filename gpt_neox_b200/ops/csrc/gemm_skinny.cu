@@ -64,9 +64,12 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
                      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// NT: groups of 8 rows of X.  U: k-blocks of a warp whose loads are issued together.
+// CTAs an SM holds of the kernel for NT groups of 8 rows of X (its accumulators and fragments take twice the registers at 4).
+constexpr int resident_ctas(int nt) { return nt == 4 ? 2 : 4; }
+
+// U: k-blocks of a warp whose loads are issued together.
 template <bool H16, int NT, int U>
-__global__ void __launch_bounds__(SK_THREADS, NT == 4 ? 2 : 4) gemm_skinny_kernel(const SkinnyParams p) {
+__global__ void __launch_bounds__(SK_THREADS, resident_ctas(NT)) gemm_skinny_kernel(const SkinnyParams p) {
     __shared__ float part[SK_WARPS][NT * 8][SK_ROWS + 1];
     __shared__ float mine[NT * 8][SK_ROWS + 1];
     cg::cluster_group cluster = cg::this_cluster();
@@ -197,8 +200,9 @@ extern "C" int neox_gemm_skinny_16(const void* A, const void* B, void* D, int M,
     e.aux = static_cast<const __nv_bfloat16*>(aux); e.ldaux = ldaux;
     e.act = act; e.alpha = alpha; e.vec_ok = 0; e.status = nullptr; e.row_ptrs = nullptr;
     const int tiles = (N + SK_ROWS - 1) / SK_ROWS, nblk = (K + SK_BK - 1) / SK_BK;
-    // Split K over a cluster while one wave (four CTAs an SM) still holds them all and no warp runs out of k-blocks.
-    const int wave = 4 * neox_sm_count();
+    // Split K over a cluster while one wave still holds them all and no warp runs out of k-blocks.  (Counting four CTAs an SM also
+    // for more than 16 rows made two waves of some products: 17 rows 2048 x 2048 9.3 us against 5.6, 2048 x 8192 16.8 / 13.3.)
+    const int wave = resident_ctas(M <= 8 ? 1 : M <= 16 ? 2 : 4) * neox_sm_count();
     int csize = 1;
     while (csize < 8 && tiles * csize * 2 <= wave && nblk >= 2 * csize * SK_WARPS) csize *= 2;
     cudaStream_t s = static_cast<cudaStream_t>(stream_);
