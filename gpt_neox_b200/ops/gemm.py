@@ -75,15 +75,19 @@ def use_pair_kernel(M, N, K):
 
 PAIR_DEFAULT = True
 SKINNY_MAX_M = 32       # csrc/gemm_skinny.cu
+SKINNY_MAX_MNK = 1.75e9
 
 
 def use_skinny_kernel(M, N, K, a_mn, b_mn):
     """The weight-streaming kernel (``csrc/gemm_skinny.cu``) takes the products of few rows with a K-major weight matrix:
-    the linear layers of a decoding step.  It reads the rows of ``a`` again for every 16 rows of ``b``, so with 17 to 32 rows
-    it only pays where the tile kernels do not fill the machine (measured at 32 rows: 2048 x 8192 25 against 57 us,
-    8192 x 2048 21 against 25, 18432 x 6144 76 against 66, 50304 x 1024 52 against 37; at 16 rows it is never slower).
+    the linear layers of a decoding step.  It reads the rows of ``a`` again for every 16 rows of ``b``, so with more than 8 rows
+    it only pays where the tile kernels do not fill the machine (N <= 8192), with 9 to 16 also while the product is small.
+    Measured, us, this kernel and the tile kernel that would run: 16 rows 12288 x 4096 31.9 / 34.2, 50304 x 2048 51.6 / 53.2,
+    18432 x 6144 52.2 / 50.1, 32000 x 4096 65.7 / 55.5; 12 rows 32000 x 4096 61.9 / 62.4, 24576 x 6144 71.8 / 63.4; 9 rows
+    50432 x 6144 129 / 128; 32 rows 2048 x 8192 14.6 / 53.2, 8192 x 2048 15.6 / 18.9, 12288 x 4096 39.1 / 34.3, 50304 x 1024
+    46.0 / 29.5; up to 8 rows it was faster everywhere (8 rows 50432 x 6144 109 / 147).
     ``NEOX_GEMM_2CTA=0/1`` forces one of the two tile kernels instead."""
-    if M > SKINNY_MAX_M or a_mn or b_mn or K % 8 or (M > 16 and N > 8192):
+    if M > SKINNY_MAX_M or a_mn or b_mn or K % 8 or (M > 8 and N > 8192 and (M > 16 or M * N * K > SKINNY_MAX_MNK)):
         return False
     use_pair_kernel(M, 1, 1)                # reads the switch
     return _PAIR not in ("0", "1")

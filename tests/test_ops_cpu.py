@@ -340,3 +340,16 @@ def test_kernels_that_start_early_use_no_read_only_loads():
             assert "ld.global.nc" not in text, path.name
         seen += len(kernels)
     assert seen >= 4
+
+
+@pytest.mark.parametrize("M,N,K,few_rows", [
+    (1, 50432, 6144, True), (8, 50432, 6144, True), (9, 12288, 4096, True), (9, 50432, 6144, False), (12, 32000, 4096, True),
+    (12, 24576, 6144, False), (16, 50304, 2048, True), (16, 18432, 6144, False), (16, 6144, 24576, True), (17, 8192, 2048, True),
+    (17, 12288, 4096, False), (32, 2048, 8192, True), (32, 50304, 1024, False), (33, 2048, 2048, False), (4, 2048, 2044, False)])
+def test_few_row_products_take_the_faster_kernel(M, N, K, few_rows, monkeypatch):
+    """Which products of few rows stream the weights: as measured on either side of the lines (8, 16 and 32 rows, 8192 columns, the
+    size of a product of 9 to 16 rows)."""
+    from gpt_neox_b200.ops import gemm as G
+    monkeypatch.setattr(G, "_PAIR", "auto")
+    assert G.use_skinny_kernel(M, N, K, False, False) == few_rows
+    assert not G.use_skinny_kernel(M, N, K, True, False) and not G.use_skinny_kernel(M, N, K, False, True)
