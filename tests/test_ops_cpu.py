@@ -353,3 +353,41 @@ def test_few_row_products_take_the_faster_kernel(M, N, K, few_rows, monkeypatch)
     monkeypatch.setattr(G, "_PAIR", "auto")
     assert G.use_skinny_kernel(M, N, K, False, False) == few_rows
     assert not G.use_skinny_kernel(M, N, K, True, False) and not G.use_skinny_kernel(M, N, K, False, True)
+
+
+def test_attention_tile_order_starts_every_tile_once(tmp_path):
+    """The order of the attention tiles: every (tile, head) exactly once, heads in groups of consecutive ones whose operands fit
+    48 MB together, heaviest tile of all heads of a group first, the last group part full."""
+    out = _run_cpp(tmp_path, r"""
+#include <algorithm>
+#include <cstdio>
+using std::min;
+#define __device__
+#define __forceinline__ inline
+static struct { int x; } blockIdx;
+#include "flash_order.cuh"
+int main() {
+    const int tiles[] = {1, 3, 16, 64}, heads[] = {1, 2, 8, 17, 256};
+    const long long bytes[] = {0, 1000, 786432, 16ll << 20, 17ll << 20, 1ll << 40};
+    for (int t : tiles) for (int h : heads) for (long long b : bytes) {
+        const TileOrder o = tile_order(t, h, b);
+        std::printf("%d %d %lld %d", t, h, b, o.group);
+        for (blockIdx.x = 0; blockIdx.x < t * h; ++blockIdx.x) {
+            int rank, head;
+            pick_tile(o, rank, head);
+            std::printf(" %d,%d", rank, head);
+        }
+        std::printf("\n");
+    }
+}""")
+    lines = out.strip().split("\n")
+    assert len(lines) == 4 * 5 * 6
+    several = 0
+    for line in lines:
+        t, h, b, group, *order = line.split()
+        t, h, b, group = int(t), int(h), int(b), int(group)
+        assert group == max(1, min(h, (48 << 20) // max(b, 1)))
+        want = [f"{rank},{head}" for g in range(0, h, group) for rank in range(t) for head in range(g, min(g + group, h))]
+        assert order == want
+        several += group < h and h % group != 0
+    assert several > 0

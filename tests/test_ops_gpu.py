@@ -1405,6 +1405,92 @@ def test_selective_scan_carries_extreme_states_between_chunks(first):
         assert bool((got[:, 1:] == first).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols,shift,rank", [(8, 0, 0), (1000, 0, 1), (50304, 0, 0), (1001, 0, 1), (1000, 1, 0)])
+def test_cross_entropy_of_extreme_16_bit_logits(cols, shift, rank, dtype, monkeypatch):
+    """Loss and gradient over one rank's share of the vocabulary: targets owned and not owned, the largest 16-bit values, rows with
+    -inf (also at the target), with nothing but -inf and with inf, where fp64 gives inf or NaN and so must the kernels.  Both
+    forms (vector loads; odd widths and unaligned rows).  Statistics in fp32 with fast exponentials (an error of some 2^-21 of
+    the exponent, at most 2^4 where it counts), gradients rounded to 16 bits."""
+    from gpt_neox_b200.parallel import cross_entropy as CE
+    torch.manual_seed(cols)
+    rows, top = 12, torch.finfo(dtype).max if dtype == torch.float16 else 1e4
+    v0 = rank * cols
+    monkeypatch.setattr(CE.mpu, "get_model_parallel_rank", lambda: rank)
+    x = (torch.randn(rows, cols, device=DEV) * 4).to(dtype)
+    tgt = torch.randint(0, cols, (rows,), device=DEV) + v0
+    tgt[0], tgt[1], tgt[2] = v0, v0 + cols - 1, v0 + cols // 2
+    tgt[3], tgt[4] = v0 + cols, v0 - 1                                        # another rank's
+    x[5, ::2] = -float("inf")
+    tgt[5] = v0 + 1
+    x[6, tgt[6] - v0] = -float("inf")
+    x[7] = -float("inf")
+    x[8, cols // 2] = float("inf")
+    x[9, 1], x[9, 2] = top, -top
+    x[10] = top
+    x[11, 3] = float("nan")
+    buf = torch.empty(rows * cols + 8, device=DEV, dtype=dtype)
+    logits = buf[shift:shift + rows * cols].view(rows, cols).copy_(x)
+    logits = logits.detach().requires_grad_()
+    g = torch.rand(rows, device=DEV) + 0.5
+    loss = CE.vocab_parallel_cross_entropy(logits, tgt)
+    grad, = torch.autograd.grad(loss, logits, g)
+    xd, owned = x.double(), (tgt >= v0) & (tgt < v0 + cols)
+    m = xd.max(1).values
+    e = (xd - m[:, None]).exp()
+    at = (tgt - v0).clamp(0, cols - 1)
+    want = e.sum(1).log() - torch.where(owned, xd.gather(1, at[:, None])[:, 0] - m, torch.zeros_like(m))
+    p = e / e.sum(1, keepdim=True)
+    p[torch.arange(rows, device=DEV), at] -= owned.double()
+    want_grad = p * g.double()[:, None]
+    nan_rows = torch.zeros(rows, dtype=torch.bool, device=DEV)
+    nan_rows[[7, 8, 11]] = True
+    assert torch.equal(want.isnan(), nan_rows) and float(want[6]) == float("inf")
+    torch.testing.assert_close(loss.double(), want, atol=2e-5, rtol=2e-5, equal_nan=True)
+    rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11           # 8 and 11 bits of significand
+    bound = (rounding + 2.0 ** -15) * want_grad.abs() + 2.0 ** -24
+    bound[torch.arange(rows, device=DEV), at] += 2.0 ** -16                  # p - 1 carries the whole error of p
+    bad = ~((grad.double() - want_grad).abs() <= bound) & ~(grad.isnan() & want_grad.isnan())
+    assert not bad.any(), (bad.nonzero()[:5].tolist(), grad[bad][:5], want_grad[bad][:5])
+
+
+@pytest.mark.parametrize("s,b,hq,hkv,d,window,dtype", [(16384, 2, 4, 4, 128, None, torch.bfloat16), (16000, 3, 3, 3, 96, None, torch.float16),
+                                                       (16384, 4, 8, 2, 128, 1000, torch.bfloat16)])
+def test_attention_in_several_head_groups_equals_head_by_head(s, b, hq, hkv, d, window, dtype):
+    """Operands that exceed the share of L2 a group of heads may take, so that the tiles of several groups (the last one part
+    full; one key head a group with grouped queries) follow each other: the same bits as one key head at a time, forward and
+    all gradients, and some rows against fp64 (a weighted mean of values, weights of 16 bits)."""
+    from gpt_neox_b200.ops import attention as A
+    torch.manual_seed(d)
+    rep = hq // hkv
+    fwd, dkv = (48 << 20) // (4 * s * d // rep), (48 << 20) // (4 * s * d * rep)
+    assert fwd < b * hq and (b * hq) % fwd and dkv < b * hkv
+    q = torch.randn(s, b, hq, d, device=DEV).to(dtype).requires_grad_()
+    k, v = (torch.randn(s, b, hkv, d, device=DEV).to(dtype).requires_grad_() for _ in range(2))
+    g = torch.randn(s, b, hq, d, device=DEV).to(dtype)
+    out = A.flash_attention(q, k, v, True, None, window)
+    grads = torch.autograd.grad(out, (q, k, v), g)
+    for i in range(b):
+        for h in range(hkv):
+            hs = slice(h * rep, (h + 1) * rep)
+            one = [t.detach()[:, i:i + 1, sl].contiguous().requires_grad_() for t, sl in ((q, hs), (k, slice(h, h + 1)), (v, slice(h, h + 1)))]
+            o1 = A.flash_attention(*one, True, None, window)
+            g1 = torch.autograd.grad(o1, one, g[:, i:i + 1, hs].contiguous())
+            assert torch.equal(out[:, i:i + 1, hs], o1)
+            for have, want, sl in zip(grads, g1, (hs, slice(h, h + 1), slice(h, h + 1))):
+                assert torch.equal(have[:, i:i + 1, sl], want)
+    rows = torch.tensor([0, 1, 127, 128, 4095, s // 2 + 3, s - 1], device=DEV)
+    keys = torch.arange(s, device=DEV)
+    banned = keys[None] > rows[:, None]
+    if window is not None:
+        banned |= keys[None] < rows[:, None] - window
+    for i, h in ((0, 0), (b - 1, hq - 1)):
+        sc = q[rows, i, h].double() @ k[:, i, h // rep].double().t() / math.sqrt(d)
+        want = sc.masked_fill(banned, -float("inf")).softmax(-1) @ v[:, i, h // rep].double()
+        _close(out[rows, i, h], want, 2e-2 if dtype == torch.bfloat16 else 4e-3, rtol=1e-2)
+    assert native.read_status() == 0
+
+
 def test_overlapped_kernels_read_what_the_launch_before_wrote():
     """A product whose second operand, and norms whose scale and bias, are results of the overlapped launch right before, many
     times over in recycled memory: the values of the same calls with a wait in between."""
