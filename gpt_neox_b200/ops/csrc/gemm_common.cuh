@@ -78,16 +78,10 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int tile, int num_m, int num_n, int nk_all) {
     TileInfo t;
     if (p.group_mode == 0) {
-        int m_blk, n_blk, part = 0, k0 = 0, k1 = nk_all;
-        if (p.splits > 1) {
-            part = tile / (num_m * num_n);
-            tile -= part * num_m * num_n;
-            k0 = (int)((long long)nk_all * part / p.splits);
-            k1 = (int)((long long)nk_all * (part + 1) / p.splits);
-        }
+        int m_blk, n_blk;
         tile_coords(tile, num_m, num_n, m_blk, n_blk);
-        t.a_m0 = m_blk * BM; t.a_k0 = k0 * BK; t.b_n0 = n_blk * BN; t.b_k0 = k0 * BK; t.n0 = n_blk * BN; t.nk = k1 - k0;
-        t.row0 = part * p.M + m_blk * BM; t.row_end = part * p.M + p.M;
+        t.a_m0 = m_blk * BM; t.a_k0 = 0; t.b_n0 = n_blk * BN; t.b_k0 = 0; t.n0 = n_blk * BN; t.nk = nk_all;
+        t.row0 = m_blk * BM; t.row_end = p.M;
     } else if (p.group_mode == 1) {
         const int4 g = __ldg(p.groups + tile);
         t.a_m0 = g.x; t.a_k0 = 0; t.n0 = g.w * BN; t.nk = nk_all;
@@ -100,6 +94,17 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int tile, int
         t.a_m0 = m_blk * BM; t.a_k0 = g.x; t.b_n0 = n_blk * BN; t.b_k0 = g.x; t.n0 = n_blk * BN; t.nk = g.y;
         t.row0 = g.z * p.M + m_blk * BM; t.row_end = g.z * p.M + p.M;
     }
+    return t;
+}
+
+// The same for one of the parts of a split contraction.
+__device__ __forceinline__ TileInfo part_info(const GemmParams& p, int tile, int num_m, int num_n, int nk_all) {
+    const int tiles = num_m * num_n, part = tile / tiles;
+    const int k0 = (int)((long long)nk_all * part / p.splits), k1 = (int)((long long)nk_all * (part + 1) / p.splits);
+    TileInfo t = tile_info(p, tile - part * tiles, num_m, num_n, k1 - k0);
+    t.a_k0 = t.b_k0 = k0 * BK;
+    t.row0 += part * p.M;
+    t.row_end += part * p.M;
     return t;
 }
 

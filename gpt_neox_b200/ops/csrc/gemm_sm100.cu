@@ -16,6 +16,7 @@
 //
 // All barrier waits are bounded (see sm100_ptx.cuh); on a time-out the kernel records a code in the
 // status word, leaves its loops, frees its tensor memory and returns.
+#include "dynamic_smem.h"
 #include "gemm_common.cuh"
 #include "launch.cuh"
 #include "neox_b200.h"
@@ -30,6 +31,10 @@ using namespace gemm;
 
 namespace {
 
+// SPLIT: the tiles are parts of a split contraction.  A form of its own, because the producer and the issuer of a tile with few
+// neighbours are a chain of latencies: with the parts' arithmetic in the common code a contraction block took 0.34 us
+// instead of 0.31 (one row of tiles, MN-major second operand).
+template <bool SPLIT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const GemmParams p) {
@@ -68,11 +73,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (p.splits > 1) launch::let_successor_start();        // add_parts_kernel, which waits for this one
+    if constexpr (SPLIT) launch::let_successor_start();        // add_parts_kernel, which waits for this one
 
     const int num_m = (p.M + BM - 1) / BM;
     const int num_n = (p.N + BN - 1) / BN;
-    const int ntiles = p.group_mode ? __ldg(p.group_ntiles) : num_m * num_n * p.splits;
+    const int ntiles = SPLIT ? num_m * num_n * p.splits : p.group_mode ? __ldg(p.group_ntiles) : num_m * num_n;
     const int nk = (p.K + BK - 1) / BK;
 
     if (warp == 0) {
@@ -82,7 +87,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             uint32_t phase = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-                const TileInfo t = tile_info(p, tile, num_m, num_n, nk);
+                const TileInfo t = SPLIT ? part_info(p, tile, num_m, num_n, nk) : tile_info(p, tile, num_m, num_n, nk);
                 for (int kb = 0; kb < t.nk; ++kb) {
                     if (!mbar_wait(&empty[stage], phase ^ 1)) {
                         atomicExch(p.status, 101);
@@ -93,7 +98,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                     uint8_t* a_dst = sA + stage * A_STAGE_BYTES;
                     uint8_t* b_dst = sB + stage * B_STAGE_BYTES;
                     if (!p.a_mn) {
-                        tma_load_2d(a_dst, &tmA, &full[stage], t.a_k0 + kb * BK, t.a_m0);
+                        tma_load_2d(a_dst, &tmA, &full[stage], (SPLIT ? t.a_k0 : 0) + kb * BK, t.a_m0);
                     } else {
 #pragma unroll
                         for (int j = 0; j < BM / 64; ++j)
@@ -101,7 +106,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                                         t.a_k0 + kb * BK);
                     }
                     if (!p.b_mn) {
-                        tma_load_2d(b_dst, &tmB, &full[stage], t.b_k0 + kb * BK, t.b_n0);
+                        tma_load_2d(b_dst, &tmB, &full[stage], (SPLIT ? t.b_k0 : 0) + kb * BK, t.b_n0);
                     } else {
 #pragma unroll
                         for (int j = 0; j < BN / 64; ++j)
@@ -140,7 +145,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
                 }
                 tc_fence_after();
                 const uint32_t tmem_d = tmem_base + buf * BN;
-                const int nk_t = tile_info(p, tile, num_m, num_n, nk).nk;
+                const int nk_t = SPLIT ? part_info(p, tile, num_m, num_n, nk).nk : p.group_mode == 2 ? __ldg(p.groups + tile).y : nk;
                 for (int kb = 0; kb < nk_t; ++kb) {
                     if (!mbar_wait(&full[stage], phase)) {
                         atomicExch(p.status, 103);
@@ -172,7 +177,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         int buf = 0;
         uint32_t bphase = 0;
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-            const TileInfo t = tile_info(p, tile, num_m, num_n, nk);
+            const TileInfo t = SPLIT ? part_info(p, tile, num_m, num_n, nk) : tile_info(p, tile, num_m, num_n, nk);
             if (!mbar_wait_warp(&tfull[buf], bphase)) {
                 if (lane == 0) atomicExch(p.status, 104);
                 break;
@@ -403,16 +408,14 @@ static int launch_tiles(const void* A, const void* B, long long lda, long long l
     if (!p.b_mn) rc = neox_make_tmap_bf16_2d(&tmB, B, p.K, p.N, ldb, BK, BN);
     else rc = neox_make_tmap_bf16_2d(&tmB, B, p.N, p.K, ldb, 64, BK);
     if (rc) return rc;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             SMEM_BYTES);
-        if (e != cudaSuccess) return NEOX_ERR_LAUNCH;
-        attr_set = true;
-    }
+    if (!(p.splits > 1 ? allow_dynamic_smem<gemm_bf16_tcgen05_kernel<true>>(SMEM_BYTES)
+                       : allow_dynamic_smem<gemm_bf16_tcgen05_kernel<false>>(SMEM_BYTES)))
+        return NEOX_ERR_LAUNCH;
     const int num_m = (p.M + BM - 1) / BM, num_n = (p.N + BN - 1) / BN;
     const long long tiles = (long long)num_m * num_n * p.splits, sms = neox_sm_count();
-    gemm_bf16_tcgen05_kernel<<<(int)(tiles < sms ? tiles : sms), NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+    const int grid = (int)(tiles < sms ? tiles : sms);
+    if (p.splits > 1) gemm_bf16_tcgen05_kernel<true><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+    else gemm_bf16_tcgen05_kernel<false><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
@@ -617,12 +620,10 @@ extern "C" int neox_gemm_grouped_16(const void* A, const void* B, void* D, int M
     if (aux) vec = vec && al16(aux) && (ldaux % 8 == 0);
     p.vec_ok = vec ? 1 : 0;
 
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SMEM_BYTES);
-    if (e != cudaSuccess) return NEOX_ERR_LAUNCH;
+    if (!allow_dynamic_smem<gemm_bf16_tcgen05_kernel<false>>(SMEM_BYTES)) return NEOX_ERR_LAUNCH;
     int grid = max_tiles;
     const int sms = neox_sm_count();
     if (grid > sms) grid = sms;
-    gemm_bf16_tcgen05_kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+    gemm_bf16_tcgen05_kernel<false><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
