@@ -155,9 +155,9 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float2 (&red)[32]
 // warp each (no barrier at all, 16 to 32 rows in flight on an SM), longer rows to a CTA with one barrier per reduction.
 // V, the vectors of 8 elements a thread holds, is a template parameter so that a thread keeps registers only for what it
 // has; with room for 4 compiled in throughout, 768-column rows ran at 18 % of the copy bandwidth backward and 20 % forward.
-// In both forms the next row is requested before this row's reductions.  8192 rows, before and now: 768 columns forward
-// 19.0 -> 8.0 us, backward with addend 44.1 -> 15.4 (7.6 of bytes); 6144 columns 83 -> 55 and 223 -> 157 (60 of bytes);
-// 4096, RMS 42 -> 24 and 158 -> 104; 5781 rows of 1024 in fp16 14.5 -> 8.3 and 30.3 -> 13.5.
+// In both forms the next row is requested before this row's reductions.  Replayed, before and now, 8192 rows: 768 columns
+// forward 17 -> 8.0 us; 6144 columns forward 55 -> 43 (31 of bytes), backward 106 -> 90 (46) and with addend 187 -> 108 (61);
+// 4096, RMS 35 -> 24, 94 -> 60 and 149 -> 81; 5781 rows of 1024 forward 14.2 -> 7.2.
 constexpr int ROW_WARPS = 8;          // rows of up to 1024 columns: warps (rows) per CTA
 constexpr int ROW_COLS = 1024;
 constexpr int CTA_THREADS = 384;      // longer rows: V = ceil(vectors / 384), 1 to 3; V = 0 re-reads the row instead
@@ -279,13 +279,15 @@ norm_fwd_kernel(const T* x, const T* gamma, const T* beta, T* y, float* __restri
 
 // Backward.  Column sums (dgamma, dbeta) are accumulated in registers (V > 0) or in global partial rows (generic path)
 // and written to partial[blockIdx.x][cols]; a second kernel reduces the partial rows.  partial layout: [2][nblk][cols]
-// fp32.  The current row stays packed between its two uses (statistics, output), which halves the registers it takes.
-template <typename T, bool RMS, int V>
+// fp32.  The current row stays packed between its two uses (statistics, output), which halves the registers it takes.  ADD is a
+// template parameter because two CTAs an SM leave 84 registers, which the addend's share and its tests overran by 40: 8192 x
+// 6144, LayerNorm, 128 us without an addend and 131 with, 90 and 108 as two forms.
+template <typename T, bool RMS, int V, bool ADD>
 __global__ void __launch_bounds__(CTA_THREADS, sizeof(T) == 2 && V < 3 ? 2 : 1)
 norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __restrict__ gamma,
                 const float* __restrict__ stat0, const float* __restrict__ stat1, T* dx, float* __restrict__ partial,
                 int rows, int cols, float eps, const T* add) {
-    // add (optional, may alias dx): dx = gradient through the norm + add -- lets the caller fold the other
+    // add (with ADD; may alias dx): dx = gradient through the norm + add -- lets the caller fold the other
     // gradient contributions of the norm's input (residual path, a sibling norm) into this pass
     __shared__ float2 red0[32], red1[32];
     constexpr bool CACHED = V > 0;
@@ -334,7 +336,7 @@ norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __res
                 cx[j] = nx[j];
                 cgr[j] = ng[j];
                 const int c = tid + j * width;
-                if (add && c < nvec) ca[j] = Vec8<T>::raw_load(add + (size_t)row * cols + c * 8);
+                if (ADD && c < nvec) ca[j] = Vec8<T>::raw_load(add + (size_t)row * cols + c * 8);
             }
             if (row + step < rows) fetch(row + step);
 #pragma unroll
@@ -394,7 +396,7 @@ norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __res
             for (int i = 0; i < 8; ++i) {
                 const float xh = RMS ? xt[i] : (xt[i] - mean) * sc, gg = gt[i] * gm[i];
                 o[i] = RMS ? gg * sc - xh * k2 : sc * (gg - k1 - xh * k2);
-                if (add) o[i] += a8[i];
+                if (ADD) o[i] += a8[i];
             }
             Vec8<T>::store(dr + c * 8, o);
         };
@@ -406,7 +408,7 @@ norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __res
                     float xt[8], gt[8], a8[8];
                     Vec8<T>::unpack(cx[j], xt);
                     Vec8<T>::unpack(cgr[j], gt);
-                    if (add) Vec8<T>::unpack(ca[j], a8);
+                    if (ADD) Vec8<T>::unpack(ca[j], a8);
                     emit(c, xt, gt, a8);
                 }
             }
@@ -415,7 +417,7 @@ norm_bwd_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* __res
                 float xt[8], gt[8], a8[8];
                 Vec8<T>::load(xr + c * 8, xt);
                 Vec8<T>::load(gr + c * 8, gt);
-                if (add) Vec8<T>::load(add + (size_t)row * cols + c * 8, a8);
+                if (ADD) Vec8<T>::load(add + (size_t)row * cols + c * 8, a8);
                 emit(c, xt, gt, a8);
             }
         }
@@ -624,9 +626,12 @@ void launch_norm_bwd_t(const void* g, const void* x, const void* gamma, const fl
         if constexpr (decltype(warp)::value)
             norm_bwd_rows_kernel<T, RMS, V><<<nblk, ROWS_THREADS, 0, st>>>((const T*)g, (const T*)x, (const T*)gamma, s0, s1,
                                                                           (T*)dx, ws, rows, cols, eps, (const T*)add);
-        else
-            norm_bwd_kernel<T, RMS, V><<<nblk, cta_threads(cols / 8, V), 0, st>>>(
+        else if (add)
+            norm_bwd_kernel<T, RMS, V, true><<<nblk, cta_threads(cols / 8, V), 0, st>>>(
                 (const T*)g, (const T*)x, (const T*)gamma, s0, s1, (T*)dx, ws, rows, cols, eps, (const T*)add);
+        else
+            norm_bwd_kernel<T, RMS, V, false><<<nblk, cta_threads(cols / 8, V), 0, st>>>(
+                (const T*)g, (const T*)x, (const T*)gamma, s0, s1, (T*)dx, ws, rows, cols, eps, nullptr);
         return 0;
     });
 }

@@ -1517,3 +1517,26 @@ def test_overlapped_kernels_read_what_the_launch_before_wrote():
             got = [step(s, False) for s in src]
             for p, q in zip(want, got):
                 assert all(torch.equal(s, t) for s, t in zip(p, q))
+
+
+@pytest.mark.parametrize("kind", ["ln", "rms"])
+@pytest.mark.parametrize("rows,cols,dtype", [(9, 520, torch.bfloat16), (700, 1032, torch.bfloat16), (9, 3080, torch.float32),
+                                             (650, 6152, torch.float16), (310, 8200, torch.bfloat16), (3, 9224, torch.bfloat16)])
+def test_norm_backward_without_addend_matches_fp64(kind, rows, cols, dtype):
+    """The backward forms without another gradient to add, through autograd: row results round once after fp32 sums, column sums are
+    fp32 over ``rows`` terms and round to the parameter's type."""
+    torch.manual_seed(rows + cols)
+    x, g = (torch.randn(rows, cols, device=DEV).to(dtype) for _ in range(2))
+    w, b = (1 + 0.1 * torch.randn(cols, device=DEV)).to(dtype), (0.1 * torch.randn(cols, device=DEV)).to(dtype)
+    ours, exact = [[t.detach().clone().requires_grad_() for t in ts] for ts in ((x, w, b), (x.double(), w.double(), b.double()))]
+    if kind == "ln":
+        y, yr = OF.layer_norm(*ours, 1e-5), torch.nn.functional.layer_norm(exact[0], (cols,), exact[1], exact[2], 1e-5)
+    else:
+        y = OF.rms_norm(*ours, 1e-5)
+        yr = exact[0] / (exact[0].pow(2).mean(-1, keepdim=True).sqrt() + 1e-5) * exact[1] + exact[2]
+    got, want = torch.autograd.grad(y, ours, g), torch.autograd.grad(yr, exact, g.double())
+    ulp = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -18}[dtype]
+    _close(y, yr, ulp, rtol=ulp)
+    _close(got[0], want[0], ulp, rtol=ulp)
+    for a, e in zip(got[1:], want[1:]):
+        _close(a, e, 1e-5 * math.sqrt(rows) + 1e-5, rtol=1e-5 + ulp)
