@@ -178,8 +178,9 @@ norm_fwd_kernel(const T* x, const T* gamma, const T* beta, T* y, float* __restri
     constexpr bool CACHED = V > 0;
     const int nvec = cols >> 3;
     const int tid = WARP ? threadIdx.x & 31 : threadIdx.x, width = WARP ? 32 : blockDim.x;
-    const int first = WARP ? blockIdx.x * ROW_WARPS + (threadIdx.x >> 5) : blockIdx.x;
-    const int step = WARP ? gridDim.x * ROW_WARPS : gridDim.x;
+    const int warps = blockDim.x >> 5;
+    const int first = WARP ? blockIdx.x * warps + (threadIdx.x >> 5) : blockIdx.x;
+    const int step = WARP ? gridDim.x * warps : gridDim.x;
     launch::let_successor_start();
     launch::wait_for_predecessor();
     typename Vec8<T>::Raw nxt[CACHED ? V : 1];
@@ -598,12 +599,22 @@ int cta_threads(int nvec, int v) { return v ? ((nvec + v - 1) / v + 31) / 32 * 3
 template <typename T, bool RMS>
 int launch_norm_fwd_t(const void* x, const void* gamma, const void* beta, void* y, float* s0, float* s1, int rows, int cols,
                       float eps, cudaStream_t st) {
+    const int sms = neox_sm_count();
+    // A warp for a row is right where there are rows for several warps on every SM.  With fewer, what counts is the latency of a
+    // row, which is shorter with one vector for each thread of a CTA.  LayerNorm in a replayed graph, warp / CTA: 1 row of 1024
+    // 2.85 / 1.74 us, 300 rows of 1024 3.31 / 2.04, 590 rows of 768 2.78 / 2.05; a row of 256 is a vector a lane either way,
+    // 1 row 1.53 / 1.69.
+    if (cols <= ROW_COLS && cols > 256 && rows < 4 * sms)
+        return launch::overlapped(norm_fwd_kernel<T, RMS, 1, false>, dim3(rows), dim3(cta_threads(cols / 8, 1)), 1, st, (const T*)x,
+                                  (const T*)gamma, (const T*)beta, (T*)y, s0, s1, rows, cols, eps);
     return for_row_length(cols, [&](auto v, auto warp) {
         constexpr int V = decltype(v)::value;
         constexpr bool WARP = decltype(warp)::value;
-        const int blocks = WARP ? (rows + ROW_WARPS - 1) / ROW_WARPS : rows, most = neox_sm_count() * 8;
+        // fewer warps a CTA before SMs stay without one
+        const int fill = (rows + sms - 1) / sms, warps = fill < ROW_WARPS ? fill : ROW_WARPS;
+        const int blocks = WARP ? (rows + warps - 1) / warps : rows, most = sms * 8;
         return launch::overlapped(norm_fwd_kernel<T, RMS, V, WARP>, dim3(blocks < most ? blocks : most),
-                                  dim3(WARP ? ROW_WARPS * 32 : cta_threads(cols / 8, V)), 1, st, (const T*)x, (const T*)gamma,
+                                  dim3(WARP ? warps * 32 : cta_threads(cols / 8, V)), 1, st, (const T*)x, (const T*)gamma,
                                   (const T*)beta, (T*)y, s0, s1, rows, cols, eps);
     });
 }
