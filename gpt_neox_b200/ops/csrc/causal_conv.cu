@@ -1,13 +1,15 @@
 // Depth-wise causal convolution over time of width 4 with bias and SiLU, channel-last, forward and backward:
 //     pre[t] = bias + sum_k w[k] * x[t - 3 + k],      out[t] = silu(pre[t]) or pre[t]
 //
-// Bound by bytes: x in, out out (backward: x and the gradient in, the gradient of x out).  A thread walks a run of time
-// steps of 8 (forward) or 4 (backward) neighbouring channels with the last three inputs in registers, so every input is
-// read once apart from the three steps in front of a run; any batch and time strides are taken, which lets the operands
-// be slices of a wider projection.  The library convolution it replaces wanted [b, d, l] (a transposing copy each way),
-// ran SiLU and the bias as passes of their own and took 168 us forward, 220 us backward at b 4, l 2048, d 1536, with
-// about 400 us of copies around them; these kernels take 27 and 62 us there (15 and 23 us of bytes).  The weight gradient is summed in registers and shared memory and
-// leaves as one partial sum per block, so results are bitwise repeatable.
+// A thread walks a run of time steps of 8 (forward) or 4 (backward) neighbouring channels with the last three inputs in
+// registers, so every input is read once apart from the three steps in front of a run (backward also three behind it); any
+// batch and time strides are taken, which lets the operands be slices of a wider projection.  The library convolution it
+// replaces wanted [b, d, l] (a transposing copy each way), ran SiLU and the bias as passes of their own and took 168 us
+// forward, 220 us backward at b 4, l 2048, d 1536, with about 400 us of copies around them; these kernels take 23 and 62 us
+// there.  Their bytes (x in, out out; backward x and the gradient in, the gradient of x out) would take 7.7 and 11.5: what
+// bounds them is the latency of a run's loads, with 20 % of an SM's warps resident at 112 and 96 registers a thread and
+// most of them waiting for memory.  The weight gradient is summed in registers and shared memory and leaves as one partial sum
+// per block, so results are bitwise repeatable.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -17,8 +19,8 @@ namespace {
 
 constexpr int W = 4;             // taps
 constexpr int TX = 32, TY = 8;   // channel groups x runs per block
-constexpr int FC = 8, FT = 16;   // forward: channels and steps of a thread
-constexpr int BC = 4, BT = 32;   // backward
+constexpr int FC = 8, FT = 16, FT_SHORT = 4;   // forward: channels and steps of a thread
+constexpr int BC = 4, BT = 32, BT_SHORT = 8;   // backward
 
 template <typename T> __device__ __forceinline__ float2 to_f2(uint32_t w);
 template <> __device__ __forceinline__ float2 to_f2<__nv_bfloat16>(uint32_t w) {
@@ -70,7 +72,7 @@ __device__ __forceinline__ void taps(const T* w, const T* bias, int c, float (&t
     }
 }
 
-template <typename T>
+template <typename T, int FT>
 __global__ void __launch_bounds__(TX * TY)
 conv_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ out, int l,
                 int d, int cblk, long long xb, long long xt, long long ob, long long ot, int silu) {
@@ -103,7 +105,7 @@ conv_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __res
 }
 
 // part: [blocks along batch and time][d][W + 1] partial sums of the tap and bias gradients
-template <typename T>
+template <typename T, int BT>
 __global__ void __launch_bounds__(TX * TY)
 conv_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, const T* __restrict__ g,
                 T* __restrict__ gx, float* __restrict__ part, int l, int d, int cblk, long long xb, long long xt,
@@ -190,7 +192,16 @@ bool aligned(const void* p, int bytes) { return (reinterpret_cast<uintptr_t>(p) 
 
 }  // namespace
 
-extern "C" int neox_causal_conv_blocks(int b, int l) { return b * ((l + BT * TY - 1) / (BT * TY)); }
+// Steps of a thread.  A run re-reads the three inputs in front of it (backward also the three steps behind it), so runs are long
+// where the machine has a block for every SM all the same, and short where a run's serial chain is all there is: forward
+// at b 1, l 128, d 512 10.8 us with the long runs and 6.8 with the short ones, both passes 29.5 and 18.7.
+static int run_length(int b, int l, int d, int channels, int run, int short_run) {
+    const long long blocks = (long long)b * ((d / channels + TX - 1) / TX) * ((l + run * TY - 1) / (run * TY));
+    return blocks < neox_sm_count() ? short_run : run;
+}
+static int time_blocks(int l, int run) { return (l + run * TY - 1) / (run * TY); }
+
+extern "C" int neox_causal_conv_blocks(int b, int l, int d) { return b * time_blocks(l, run_length(b, l, d, BC, BT, BT_SHORT)); }
 
 // strides: element strides (batch, time) of x and out; d and the strides multiples of 8.  w: [d][4].  bias may be NULL.
 extern "C" int neox_causal_conv_fwd(const void* x, const void* w, const void* bias, void* out, const long long* strides, int b,
@@ -200,19 +211,24 @@ extern "C" int neox_causal_conv_fwd(const void* x, const void* w, const void* bi
     for (int i = 0; i < 4; ++i)
         if (strides[i] % 8) return NEOX_ERR_ALIGN;
     if (!aligned(x, 16) || !aligned(out, 16)) return NEOX_ERR_ALIGN;
-    const int cblk = (d / FC + TX - 1) / TX, tblk = (l + FT * TY - 1) / (FT * TY);
+    const int run = run_length(b, l, d, FC, FT, FT_SHORT), cblk = (d / FC + TX - 1) / TX, tblk = time_blocks(l, run);
     dim3 grid(cblk * tblk, b), block(TX, TY);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define CONV_FWD(T)                                                                                                      \
-    conv_fwd_kernel<T><<<grid, block, 0, s>>>((const T*)x, (const T*)w, (const T*)bias, (T*)out, l, d, cblk, strides[0], \
-                                              strides[1], strides[2], strides[3], silu)
-    if (h16) CONV_FWD(__half);
-    else CONV_FWD(__nv_bfloat16);
+#define CONV_FWD(T, RUN)                                                                                                      \
+    conv_fwd_kernel<T, RUN><<<grid, block, 0, s>>>((const T*)x, (const T*)w, (const T*)bias, (T*)out, l, d, cblk, strides[0], \
+                                                   strides[1], strides[2], strides[3], silu)
+    if (run == FT) {
+        if (h16) CONV_FWD(__half, FT);
+        else CONV_FWD(__nv_bfloat16, FT);
+    } else {
+        if (h16) CONV_FWD(__half, FT_SHORT);
+        else CONV_FWD(__nv_bfloat16, FT_SHORT);
+    }
 #undef CONV_FWD
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
-// strides: of x, g (gradient of out) and gx.  part: neox_causal_conv_blocks(b, l) x d x 5 floats (4 taps, bias).
+// strides: of x, g (gradient of out) and gx.  part: neox_causal_conv_blocks(b, l, d) x d x 5 floats (4 taps, bias).
 extern "C" int neox_causal_conv_bwd(const void* x, const void* w, const void* bias, const void* g, void* gx, float* part,
                                     const long long* strides, int b, int l, int d, int silu, int h16, void* stream) {
     if (b <= 0 || l <= 0 || d <= 0) return 0;
@@ -220,15 +236,20 @@ extern "C" int neox_causal_conv_bwd(const void* x, const void* w, const void* bi
     for (int i = 0; i < 6; ++i)
         if (strides[i] % 8) return NEOX_ERR_ALIGN;
     if (!aligned(x, 8) || !aligned(g, 8) || !aligned(gx, 8)) return NEOX_ERR_ALIGN;
-    const int cblk = (d / BC + TX - 1) / TX, tblk = (l + BT * TY - 1) / (BT * TY);
+    const int run = run_length(b, l, d, BC, BT, BT_SHORT), cblk = (d / BC + TX - 1) / TX, tblk = time_blocks(l, run);
     dim3 grid(cblk * tblk, b), block(TX, TY);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define CONV_BWD(T)                                                                                                       \
-    conv_bwd_kernel<T><<<grid, block, 0, s>>>((const T*)x, (const T*)w, (const T*)bias, (const T*)g, (T*)gx, part, l, d,  \
-                                              cblk, strides[0], strides[1], strides[2], strides[3], strides[4], strides[5], \
-                                              silu)
-    if (h16) CONV_BWD(__half);
-    else CONV_BWD(__nv_bfloat16);
+#define CONV_BWD(T, RUN)                                                                                                       \
+    conv_bwd_kernel<T, RUN><<<grid, block, 0, s>>>((const T*)x, (const T*)w, (const T*)bias, (const T*)g, (T*)gx, part, l, d,  \
+                                                   cblk, strides[0], strides[1], strides[2], strides[3], strides[4], strides[5], \
+                                                   silu)
+    if (run == BT) {
+        if (h16) CONV_BWD(__half, BT);
+        else CONV_BWD(__nv_bfloat16, BT);
+    } else {
+        if (h16) CONV_BWD(__half, BT_SHORT);
+        else CONV_BWD(__nv_bfloat16, BT_SHORT);
+    }
 #undef CONV_BWD
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }

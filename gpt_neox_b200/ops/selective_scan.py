@@ -156,7 +156,7 @@ class _CausalConv(torch.autograd.Function):
             else torch.empty(b, l, width, dtype=xz.dtype, device=xz.device)
         if width > d:
             gxz[..., d:].copy_(gz)
-        part = torch.empty(native.lib().neox_causal_conv_blocks(b, l), d, w.shape[1] + 1, dtype=torch.float32, device=xz.device)
+        part = torch.empty(native.lib().neox_causal_conv_blocks(b, l, d), d, w.shape[1] + 1, dtype=torch.float32, device=xz.device)
         rc = native.lib().neox_causal_conv_bwd(native.ptr(xz), native.ptr(w), native.ptr(bias), native.ptr(g),
                                                native.ptr(gxz), native.ptr(part), _strides(xz, g, gxz), b, l, d,
                                                int(ctx.silu), int(xz.dtype == torch.float16),

@@ -1540,3 +1540,18 @@ def test_norm_backward_without_addend_matches_fp64(kind, rows, cols, dtype):
     _close(got[0], want[0], ulp, rtol=ulp)
     for a, e in zip(got[1:], want[1:]):
         _close(a, e, 1e-5 * math.sqrt(rows) + 1e-5, rtol=1e-5 + ulp)
+
+
+@pytest.mark.parametrize("b,l,d", [(5, 2053, 520), (1, 40, 16), (2, 300, 1032)])
+def test_causal_conv_long_and_short_runs(b, l, d):
+    """Runs of 16 / 32 steps, where the machine is full with them, and of 4 / 8: outputs and all gradients against the library
+    convolution in fp32.  Outputs round once; the weight gradient rounds once after b l fp32 products."""
+    from gpt_neox_b200.ops import selective_scan as SS
+    torch.manual_seed(l)
+    leaves = [torch.randn(b, l, d, device=DEV).to(torch.bfloat16), (torch.randn(d, 4, device=DEV) * 0.5).to(torch.bfloat16),
+              torch.randn(d, device=DEV).to(torch.bfloat16)]
+    g = torch.randn(b, l, d, device=DEV).to(torch.bfloat16)
+    ours, ref = [[t.to(ty).requires_grad_() for t in leaves] for ty in (torch.bfloat16, torch.float64)]
+    y, yr = SS.causal_conv1d(*ours), SS.causal_conv1d(*ref)
+    for a, e in zip([y, *torch.autograd.grad(y, ours, g)], [yr, *torch.autograd.grad(yr, ref, g.double())]):
+        _close(a, e, 2e-4 + 2.0 ** -9 * e.abs().mean().item(), rtol=2.0 ** -8)
