@@ -519,13 +519,14 @@ template <typename T> __device__ __forceinline__ void unpack_8(const uint4& u, f
 
 // Single-pass (online) statistics for 16-bit logits with cols % 8 == 0: one sweep of 16-byte loads keeps a running
 // (max, sum of exp relative to that max) per thread, merged across the CTA at the end.
-//   row_max[row] = max_c x,   stats[row] = (sum_c exp(x - row_max), x[target - v0] (raw) if owned else 0)
-// The caller turns these local quantities into global ones after the tensor-parallel all-reduce of the maxima.
+//   row_max[row] = max_c x,   stats[row] = (sum_c exp(x - row_max), x[target - v0] if owned else 0)
+// relative: the target logit less row_max, as the loss wants it.  Else it is raw, for a vocabulary that is split over ranks:
+// ce_rebase_kernel turns the local quantities into global ones after the all-reduce of the maxima.
 template <typename T>
 __global__ void __launch_bounds__(256) ce_online_kernel(const T* __restrict__ x,
                                                              const long long* __restrict__ target,
                                                              float* __restrict__ row_max, float* __restrict__ stats,
-                                                             int rows, int cols, int v0) {
+                                                             int rows, int cols, int v0, int relative) {
     __shared__ float red_m[8], red_s[8];
     const int nvec = cols >> 3;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -569,9 +570,21 @@ __global__ void __launch_bounds__(256) ce_online_kernel(const T* __restrict__ x,
             const long long t = target[row] - v0;
             row_max[row] = gm;
             stats[2 * row] = gs;
-            stats[2 * row + 1] = (t >= 0 && t < cols) ? to_f<T>(x[(size_t)row * cols + t]) : 0.f;
+            stats[2 * row + 1] = (t >= 0 && t < cols) ? to_f<T>(x[(size_t)row * cols + t]) - (relative ? gm : 0.f) : 0.f;
         }
     }
+}
+
+// stats[row] (local) <- relative to the maximum over all ranks.  One thread a row; the exponential in fp64, as its argument may be
+// large and a row has one.
+__global__ void __launch_bounds__(256) ce_rebase_kernel(const long long* __restrict__ target, const float* __restrict__ local_max,
+                                                        const float* __restrict__ row_max, float* __restrict__ stats, int rows,
+                                                        int cols, int v0) {
+    const int row = blockIdx.x * 256 + threadIdx.x;
+    if (row >= rows) return;
+    const long long t = target[row] - v0;
+    stats[2 * row] *= (float)exp((double)(local_max[row] - row_max[row]));
+    stats[2 * row + 1] = (t >= 0 && t < cols) ? stats[2 * row + 1] - row_max[row] : 0.f;
 }
 
 // Vectorised backward for 16-bit logits, cols % 8 == 0 (same math as ce_bwd_kernel).
@@ -981,18 +994,26 @@ int neox_ce_stats(const void* x, const long long* target, const float* row_max, 
                                                                        cols, v0)));
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
-// bf16 only, cols % 8 == 0: local row maximum, sum of exp relative to it, and the raw target logit in one pass.
+// bf16 (0) or fp16 (2), cols % 8 == 0: local row maximum, sum of exp relative to it, and the target logit, relative to it too or
+// raw, in one pass.
 int neox_ce_online_16(const void* x, const long long* target, float* row_max, float* stats, int rows, int cols,
-                      int v0, int dtype, void* stream) {
+                      int v0, int dtype, int relative, void* stream) {
     if (rows <= 0) return 0;
     if (dtype != 0 && dtype != 2) return NEOX_ERR_SHAPE;
     if (cols % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return NEOX_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == 0)
         ce_online_kernel<__nv_bfloat16><<<row_grid(rows), 256, 0, st>>>((const __nv_bfloat16*)x, target, row_max, stats, rows,
-                                                                       cols, v0);
+                                                                       cols, v0, relative);
     else
-        ce_online_kernel<__half><<<row_grid(rows), 256, 0, st>>>((const __half*)x, target, row_max, stats, rows, cols, v0);
+        ce_online_kernel<__half><<<row_grid(rows), 256, 0, st>>>((const __half*)x, target, row_max, stats, rows, cols, v0, relative);
+    return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
+}
+// What neox_ce_online_16 left raw, relative to row_max, the maximum over all ranks.
+int neox_ce_rebase(const long long* target, const float* local_max, const float* row_max, float* stats, int rows, int cols, int v0,
+                   void* stream) {
+    if (rows <= 0) return 0;
+    ce_rebase_kernel<<<(rows + 255) / 256, 256, 0, (cudaStream_t)stream>>>(target, local_max, row_max, stats, rows, cols, v0);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 int neox_ce_bwd(const void* x, const long long* target, const float* row_max, const float* stats, const float* g,

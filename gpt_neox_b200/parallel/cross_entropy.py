@@ -69,16 +69,14 @@ class _VocabParallelCE(torch.autograd.Function):
             row_max = torch.empty(rows, dtype=torch.float32, device=logits2.device)
             stats = torch.empty(rows, 2, dtype=torch.float32, device=logits2.device)
             rc = native.lib().neox_ce_online_16(native.ptr(logits2), native.ptr(tgt), native.ptr(row_max),
-                                                native.ptr(stats), rows, vloc, v0, _DT[logits2.dtype], _s())
+                                                native.ptr(stats), rows, vloc, v0, _DT[logits2.dtype], int(tp == 1), _s())
             native.check(rc, "neox_ce_online_16")
-            local_max = row_max
             if tp > 1:
-                row_max = local_max.clone()
+                local_max, row_max = row_max, row_max.clone()
                 dist.all_reduce(row_max, op=dist.ReduceOp.MAX, group=mpu.get_model_parallel_group())
-                stats[:, 0] *= torch.exp(local_max - row_max)
-            local_t = tgt - v0
-            owned = (local_t >= 0) & (local_t < vloc)
-            stats[:, 1] = torch.where(owned, stats[:, 1] - row_max, torch.zeros_like(row_max))
+                rc = native.lib().neox_ce_rebase(native.ptr(tgt), native.ptr(local_max), native.ptr(row_max),
+                                                 native.ptr(stats), rows, vloc, v0, _s())
+                native.check(rc, "neox_ce_rebase")
         else:
             row_max = _row_max(logits2)
             if tp > 1:

@@ -1555,3 +1555,25 @@ def test_causal_conv_long_and_short_runs(b, l, d):
     y, yr = SS.causal_conv1d(*ours), SS.causal_conv1d(*ref)
     for a, e in zip([y, *torch.autograd.grad(y, ours, g)], [yr, *torch.autograd.grad(yr, ref, g.double())]):
         _close(a, e, 2e-4 + 2.0 ** -9 * e.abs().mean().item(), rtol=2.0 ** -8)
+
+
+def test_loss_statistics_of_a_split_vocabulary():
+    """Raw statistics of one rank's share, rebased on a larger maximum: the formula in fp64 (one rounding of each factor), rows whose
+    own share is all -inf, targets of other ranks."""
+    torch.manual_seed(0)
+    rows, cols, v0 = 300, 1000, 2000
+    x = (torch.randn(rows, cols, device=DEV) * 3).to(torch.float16)
+    x[7] = -float("inf")
+    tgt = torch.randint(0, 3 * cols, (rows,), device=DEV) + 1000
+    local, stats = torch.empty(rows, device=DEV), torch.empty(rows, 2, device=DEV)
+    L = native.lib()
+    native.check(L.neox_ce_online_16(native.ptr(x), native.ptr(tgt), native.ptr(local), native.ptr(stats), rows, cols, v0, 2, 0, OF._s()), "online")
+    raw, top = stats.clone(), torch.maximum(local, torch.randn(rows, device=DEV) * 20)
+    native.check(L.neox_ce_rebase(native.ptr(tgt), native.ptr(local), native.ptr(top), native.ptr(stats), rows, cols, v0, OF._s()), "rebase")
+    owned = (tgt >= v0) & (tgt < v0 + cols)
+    assert 50 < int(owned.sum()) < 250
+    picked = x.float()[torch.arange(rows, device=DEV), (tgt - v0).clamp(0, cols - 1)]
+    assert torch.equal(raw[:, 1], torch.where(owned, picked, torch.zeros_like(picked)))
+    _close(stats[:, 0], raw[:, 0].double() * (local - top).double().exp(), 0.0, rtol=2.0 ** -22)
+    assert torch.equal(stats[:, 1], torch.where(owned, raw[:, 1] - top, torch.zeros_like(top)))
+    assert float(stats[7, 0]) == 0.0
