@@ -346,14 +346,14 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(const T* __restrict__ x, 
 }
 
 // In-place rotary embedding of the first `rot` dims of every head of q and k (views of one packed QKV tensor): one
-// thread owns the pair (e, e + rot/2), so nothing is read after it was overwritten.  cs / sn: [s, rot] fp32.
-// The same rotation, VEC elements of each half per access.  Bound by the bytes of the rotated parts, read and written in
-// place.  One element per thread, the general form below, made it 16-bit accesses and 64-bit divisions: 38.7 us for 8192
+// thread owns the pairs (e, e + rot/2), so nothing is read after it was overwritten.  cs / sn: [s, rot] fp32.
+//
+// This form takes VEC elements of each half per access.  Bound by the bytes of the rotated parts, read and written in
+// place.  One pair per thread, the general form below, makes it 16-bit accesses and 64-bit divisions: 38.7 us for 8192
 // tokens x 24 heads of 64, whole heads rotated (8 us of bytes), 117 us for 8192 x 128 heads of 96, 24 rotated.  A thread
 // keeps its piece of the fp32 tables, which is twice the size of the elements it rotates, for ROPE_HEADS heads.
 // The two shapes take 13.8 and 53.8 us here.
-constexpr int ROPE_HEADS = 4;
-template <typename T, int VEC>
+template <typename T, int VEC, int ROPE_HEADS>
 __global__ void __launch_bounds__(256) rope_qk_inplace_vec_kernel(T* __restrict__ q, T* __restrict__ k,
                                                                   const float* __restrict__ cs,
                                                                   const float* __restrict__ sn, int s, int b, int hq, int hk,
@@ -407,6 +407,7 @@ __global__ void __launch_bounds__(256) rope_qk_inplace_vec_kernel(T* __restrict_
     }
 }
 
+// One pair per thread: any width and alignment, and sizes too small to fill the machine otherwise.
 template <typename T>
 __global__ void __launch_bounds__(256) rope_qk_inplace_kernel(T* __restrict__ q, T* __restrict__ k,
                                                               const float* __restrict__ cs, const float* __restrict__ sn,
@@ -952,26 +953,38 @@ int neox_rope_qk_inplace(void* q, void* k, const float* cs, const float* sn, int
     if (total <= 0) return 0;
     if (rot % 2) return NEOX_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
-    // Vectors of 8 or 4 elements where every vector of both halves of every head starts on a multiple of its size.
+    // Vectors of 8 or 4 elements where every vector of both halves of every head starts on a multiple of its size, and there is
+    // more than an element for each of 1024 threads on every SM (512 tokens x 16 heads of 16: 2.3 us an element a thread, 2.9 in
+    // vectors, 5.5 in vectors of four heads).
     const int half = rot / 2;
     const long long strides = q_ss | q_sb | q_sh | k_ss | k_sb | k_sh;
     const uintptr_t base = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k);
     auto fits = [&](int vec) { return half % vec == 0 && strides % vec == 0 && base % (vec * 2) == 0; };
-    const int vec = dtype == 1 ? 0 : fits(8) ? 8 : fits(4) ? 4 : 0;
+    const long long full = 1024ll * neox_sm_count();
+    const int vec = dtype == 1 || total < full ? 0 : fits(8) ? 8 : fits(4) ? 4 : 0;
     if (vec) {
-        const long long items = (long long)s * b * (half / vec) * ((hq + hk + ROPE_HEADS - 1) / ROPE_HEADS);
-        const long long blocks = (items + 255) / 256;
+        // Four heads a thread where that leaves as many (2048 tokens x 24 heads of 64: 5.8 us with one, 6.8 with four).
+        const long long pieces = (long long)s * b * (half / vec), heads4 = (hq + hk + 3) / 4;
+        const int per = pieces * heads4 >= full ? 4 : 1;
+        const long long items = pieces * (per == 4 ? heads4 : hq + hk), blocks = (items + 255) / 256;
         if (blocks <= 0x7fffffff) {
-#define ROPE_VEC(T, V)                                                                                                   \
-    rope_qk_inplace_vec_kernel<T, V><<<(int)blocks, 256, 0, st>>>((T*)q, (T*)k, cs, sn, s, b, hq, hk, rot, q_ss, q_sb, q_sh, \
-                                                                  k_ss, k_sb, k_sh, inverse)
+#define ROPE_VEC(T, V, H)                                                                                                   \
+    rope_qk_inplace_vec_kernel<T, V, H><<<(int)blocks, 256, 0, st>>>((T*)q, (T*)k, cs, sn, s, b, hq, hk, rot, q_ss, q_sb,    \
+                                                                     q_sh, k_ss, k_sb, k_sh, inverse)
+#define ROPE_WIDTH(T)                       \
+    if (vec == 8) {                         \
+        if (per == 4) ROPE_VEC(T, 8, 4);    \
+        else ROPE_VEC(T, 8, 1);             \
+    } else {                                \
+        if (per == 4) ROPE_VEC(T, 4, 4);    \
+        else ROPE_VEC(T, 4, 1);             \
+    }
             if (dtype == 0) {
-                if (vec == 8) ROPE_VEC(__nv_bfloat16, 8);
-                else ROPE_VEC(__nv_bfloat16, 4);
+                ROPE_WIDTH(__nv_bfloat16)
             } else {
-                if (vec == 8) ROPE_VEC(__half, 8);
-                else ROPE_VEC(__half, 4);
+                ROPE_WIDTH(__half)
             }
+#undef ROPE_WIDTH
 #undef ROPE_VEC
             return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
         }

@@ -1577,3 +1577,33 @@ def test_loss_statistics_of_a_split_vocabulary():
     _close(stats[:, 0], raw[:, 0].double() * (local - top).double().exp(), 0.0, rtol=2.0 ** -22)
     assert torch.equal(stats[:, 1], torch.where(owned, raw[:, 1] - top, torch.zeros_like(top)))
     assert float(stats[7, 0]) == 0.0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("s,b,hq,hk,d,rot", [(2049, 1, 5, 5, 64, 64), (9001, 2, 5, 2, 64, 64), (9001, 1, 3, 1, 96, 24), (33001, 1, 5, 2, 96, 24)])
+def test_rope_in_place_vectors_of_one_and_four_heads(s, b, hq, hk, d, rot, dtype):
+    """Sizes that take the vector forms (8 and 4 elements; one and four heads a thread, the last group part full): the bits of the
+    element-wise form, which a slice of fewer tokens takes, and the rest of the projection untouched."""
+    import ctypes
+    torch.manual_seed(rot)
+    packed = torch.randn(s, b, hq + 2 * hk, d, device=DEV).to(dtype)
+    cos, sin = torch.randn(s, rot, device=DEV), torch.randn(s, rot, device=DEV)
+    ll = ctypes.c_longlong
+
+    def run(p, c, sn, inverse):
+        q, k = p[:, :, :hq], p[:, :, hq:hq + hk]
+        native.check(native.lib().neox_rope_qk_inplace(
+            native.ptr(q), native.ptr(k), native.ptr(c), native.ptr(sn), p.shape[0], b, hq, hk, rot, ll(q.stride(0)),
+            ll(q.stride(1)), ll(q.stride(2)), ll(k.stride(0)), ll(k.stride(1)), ll(k.stride(2)), inverse, OF._DT[dtype],
+            OF._s()), "rope")
+    for inverse in (0, 1):
+        whole, parts = packed.clone(), packed.clone()
+        run(whole, cos, sin, inverse)
+        for i in range(0, s, 997):
+            run(parts[i:i + 997], cos[i:i + 997], sin[i:i + 997], inverse)
+        want = OF.rope_ref(packed[:, :, :hq + hk], cos.view(s, 1, 1, rot), (-sin if inverse else sin).view(s, 1, 1, rot))
+        # one rounding after two products that may cancel
+        _close(whole[:, :, :hq + hk], want, 2.0 ** -7, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+        assert ((whole != parts).float().mean().item()) < 1e-3          # the two forms may contract the products differently
+        assert torch.equal(whole[:, :, hq + hk:], packed[:, :, hq + hk:])
+        assert torch.equal(whole[..., rot:], packed[..., rot:])
