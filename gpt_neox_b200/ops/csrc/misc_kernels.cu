@@ -617,8 +617,9 @@ __global__ void __launch_bounds__(256) ce_bwd_16_kernel(const T* __restrict__ x,
 
 // ------------------------------------------------------------------ optimizers
 // Adam over a flat shard, in place.  Bound by bytes: four fp32 streams in, three out and the 16-bit copy, 30 per element.
-// VEC = 4: one 16-byte access per stream and thread, without keeping any of it in the caches; with 4-byte accesses the
-// same pass ran at 4.8 TB/s over 1.5e9 elements and 5.4 TB/s over 0.7e9 and now at 5.4 and 5.7 TB/s.
+// VEC = 4: one 16-byte access per stream and thread, and a block for every 1024 elements.  Out of cold caches, us, 4-byte
+// accesses / 16-byte ones over a grid of 8 blocks an SM with streaming hints / this: 20e6 elements 104 / 105 / 93, 125e6
+// 619 / 645 / 547, 1.5e9 8164 / 7599 / 6477 (7.0 TB/s).
 template <typename OUT, int VEC>
 __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                                                    const float* __restrict__ g, OUT* __restrict__ out, long long n,
@@ -642,17 +643,17 @@ __global__ void __launch_bounds__(256) adam_kernel(float* __restrict__ p, float*
             OUT v[4];
         };
         for (long long i = first; i < nvec; i += stride) {
-            const float4 gv = __ldcs(reinterpret_cast<const float4*>(g) + i);
-            float4 pv = __ldcs(reinterpret_cast<const float4*>(p) + i);
-            float4 mv = __ldcs(reinterpret_cast<const float4*>(m) + i);
-            float4 vv = __ldcs(reinterpret_cast<const float4*>(v) + i);
+            const float4 gv = reinterpret_cast<const float4*>(g)[i];
+            float4 pv = reinterpret_cast<const float4*>(p)[i];
+            float4 mv = reinterpret_cast<const float4*>(m)[i];
+            float4 vv = reinterpret_cast<const float4*>(v)[i];
             update(gv.x, pv.x, mv.x, vv.x);
             update(gv.y, pv.y, mv.y, vv.y);
             update(gv.z, pv.z, mv.z, vv.z);
             update(gv.w, pv.w, mv.w, vv.w);
-            __stcs(reinterpret_cast<float4*>(m) + i, mv);
-            __stcs(reinterpret_cast<float4*>(v) + i, vv);
-            __stcs(reinterpret_cast<float4*>(p) + i, pv);
+            reinterpret_cast<float4*>(m)[i] = mv;
+            reinterpret_cast<float4*>(v)[i] = vv;
+            reinterpret_cast<float4*>(p)[i] = pv;
             if (out) {
                 Pack o;
                 o.v[0] = from_f<OUT>(pv.x);
@@ -1053,9 +1054,11 @@ int neox_adam_step(float* p, float* m, float* v, const float* g, void* out, int 
     cudaStream_t st = (cudaStream_t)stream;
     auto aligned = [](const void* q, int bytes) { return (reinterpret_cast<uintptr_t>(q) & (bytes - 1)) == 0; };
     // a shard may start anywhere in a flat buffer: four elements at a time only where all of its tensors allow it
-    const bool vec = aligned(p, 16) && aligned(m, 16) && aligned(v, 16) && aligned(g, 16) &&
+    // and there are enough of them for 1024 threads on every SM (1e5 elements: 3.1 us one at a time, 3.6 in fours)
+    const bool vec = n >= 4096ll * neox_sm_count() && aligned(p, 16) && aligned(m, 16) && aligned(v, 16) && aligned(g, 16) &&
                      (!out || aligned(out, out_dtype == 1 ? 16 : 8));
-    const int grid = grid_for(vec ? (n + 3) / 4 : n, vec ? 8 : 16);
+    const long long blocks = (n / 4 + 255) / 256;
+    const int grid = vec ? (int)(blocks < 0x7fffffff ? blocks : 0x7fffffff) : grid_for(n, 16);
 #define ADAM(T, VEC) \
     adam_kernel<T, VEC><<<grid, 256, 0, st>>>(p, m, v, g, (T*)out, n, lr, b1, b2, eps, wd, bc1, bc2, gs, adamw)
 #define ADAM_T(T) \

@@ -1607,3 +1607,29 @@ def test_rope_in_place_vectors_of_one_and_four_heads(s, b, hq, hk, d, rot, dtype
         assert ((whole != parts).float().mean().item()) < 1e-3          # the two forms may contract the products differently
         assert torch.equal(whole[:, :, hq + hk:], packed[:, :, hq + hk:])
         assert torch.equal(whole[..., rot:], packed[..., rot:])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,offset", [(700000, 0), (700003, 4), (700003, 1), (700001, 2)])
+def test_adam_vectors_equal_single_elements(n, offset, dtype):
+    """Shards large enough for four elements at a time, aligned and not, against the update in fp64 and nothing outside the shard."""
+    import ctypes
+    torch.manual_seed(n)
+    full = n + offset + 8
+    p, m, g = (torch.randn(full, device=DEV) for _ in range(3))
+    v, out = torch.rand(full, device=DEV), torch.zeros(full, device=DEV, dtype=dtype)
+    keep = [t.clone() for t in (p, m, v, out)]
+    sl = slice(offset, offset + n)
+    f = ctypes.c_float
+    native.check(native.lib().neox_adam_step(
+        native.ptr(p[sl]), native.ptr(m[sl]), native.ptr(v[sl]), native.ptr(g[sl]), native.ptr(out[sl]), OF._DT[dtype],
+        ctypes.c_longlong(n), f(1e-2), f(0.9), f(0.95), f(1e-8), f(0.1), f(0.1), f(0.05), f(0.5), 1, OF._s()), "adam")
+    P, M, V, Gr = (t[sl].double() for t in (*keep[:3], g))
+    Gr = Gr * 0.5
+    M, V = 0.9 * M + 0.1 * Gr, 0.95 * V + 0.05 * Gr * Gr
+    P = P - (1e-2 / 0.1 * M / (V.sqrt() / 0.05 ** 0.5 + 1e-8) + 1e-2 * 0.1 * P)
+    for have, want in ((p, P), (m, M), (v, V)):
+        _close(have[sl], want, 1e-6, rtol=2e-6)
+    assert torch.equal(out[sl], p[sl].to(dtype))
+    for have, was in zip((p, m, v, out), keep):
+        assert torch.equal(have[:offset], was[:offset]) and torch.equal(have[offset + n:], was[offset + n:])
