@@ -101,15 +101,10 @@ scan_state_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const
     sumd[((size_t)b * nchk + ck) * d + c] = total;
 }
 
-// h * 2^x + add: the state that a chunk of decay 2^x hands on.  The decay of 32 steps may leave the range of fp32 although the
-// state, taken step by step, does not: then it is applied in two halves.  A state of 0 stays 0 and one that has overflowed stays
-// so.
-__device__ __forceinline__ float carry(float h, float x, float add) {
-    if (fabsf(x) < 126.f) return __fmaf_rn(exp2f(x), h, add);
-    if (h == 0.f || isinf(h)) return h + add;
-    const float half = exp2f(0.5f * x);
-    return __fmaf_rn(half * h, half, add);
-}
+// An exponent as far as 2^x stays a normal number.  The decay of 32 steps may leave the range of fp32 although the state, taken
+// step by step, does not: what is left of the exponent is then applied as a second factor, which is 1 otherwise.  Neither
+// factor is ever 0 or inf, so a state of 0 stays 0 and one that has overflowed stays so.
+__device__ __forceinline__ float within_range(float x) { return fminf(fmaxf(x, -126.f), 126.f); }
 
 // ------------------------------------------------------------------ combine over the chunks, in place
 // Forward: slot k + 1 holds the state that chunk k adds; afterwards the state at the start of chunk k + 1.
@@ -122,20 +117,21 @@ scan_combine_kernel(const float* __restrict__ A, const float* __restrict__ sumd,
     const float a = A[(size_t)c * NS + j] * LOG2E;
     float h = 0.f;
     for (int k0 = 0; k0 < nchk - 1; k0 += GROUP) {
-        float loc[GROUP], dec[GROUP];
+        float loc[GROUP], x[GROUP];
 #pragma unroll
         for (int i = 0; i < GROUP; ++i) {
             if (k0 + i < nchk - 1) {
                 const int k = REVERSE ? nchk - 1 - (k0 + i) : k0 + i;
                 loc[i] = st[slot(b, REVERSE ? k - 1 : k + 1, nchk, d) + (size_t)j * d + c];
-                dec[i] = a * sumd[((size_t)b * nchk + k) * d + c];
+                x[i] = sumd[((size_t)b * nchk + k) * d + c];
             }
         }
 #pragma unroll
         for (int i = 0; i < GROUP; ++i) {
             if (k0 + i < nchk - 1) {
                 const int k = REVERSE ? nchk - 1 - (k0 + i) : k0 + i;
-                h = carry(h, dec[i], loc[i]);
+                const float e = a * x[i], e1 = within_range(e);
+                h = __fmaf_rn(exp2f(e1), exp2f(within_range(e - e1)) * h, loc[i]);
                 st[slot(b, REVERSE ? k - 1 : k + 1, nchk, d) + (size_t)j * d + c] = h;
             }
         }
