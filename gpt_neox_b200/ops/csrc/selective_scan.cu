@@ -467,11 +467,15 @@ scan_grad_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const 
     }
 }
 
-// Chunks side by side, or all chunks of a channel in one block?  Side by side costs the exponentials twice, so it is
-// left where the channels alone fill the machine: 8 blocks of 128 on every SM.
+// Chunks side by side, or all chunks of a channel in one block?  Side by side costs the exponentials twice and two launches
+// more, and pays where the blocks of 128 channels alone leave the machine idle.  Measured at 148 SMs: a block that walks all of
+// time takes 0.28 us a step, and a little longer with more of them (0.28 + 0.0005 a block up to four an SM); side by side a
+// block's chunk takes 0.053 us of the machine, and the launches some 20.  Equating the two gives the line below, r blocks an
+// SM.  In one block / side by side, us: 16 blocks 2048 steps 565 / 74, 144 blocks 512 steps 173 / 136, 221 blocks 512 steps
+// 204 / 199, 288 blocks 2048 steps 804 / 994, 592 blocks 256 steps 149 / 257, 4 blocks 64 steps 21 / 22.
 int forward_span(int b, int d, int nchk) {
-    const long long blocks = (long long)b * ((d + THREADS - 1) / THREADS);
-    return nchk == 1 || blocks >= 8ll * neox_sm_count() ? nchk : 1;
+    const double r = (double)b * ((d + THREADS - 1) / THREADS) / neox_sm_count();
+    return nchk * (9.0 - 5.5 * r) > 20.0 ? 1 : nchk;
 }
 
 Strides make_strides(const long long* s, int operands) {
