@@ -7,7 +7,7 @@
 // 59 against 50 and 49).  The tiles of a head read the same keys and values, so the order is kept within groups of heads
 // whose operands stay in L2 together (48 of 126 MB, leaving room for what the CTAs write).  48 heads of 64,
 // 2048 rows, forward / dK, dV / dQ: 91 / 125 / 99 -> 75 / 114 / 87 us; 48 of 128, 777 rows, forward 43 -> 35 us; 256 heads of
-// 96, in five groups, as before.
+// 96, in four groups, as before.
 #pragma once
 
 struct TileOrder {

@@ -3,8 +3,8 @@
 // Who needs it: callers that cannot obtain device memory at the time of the call -- a process whose GPU
 // memory is already entirely reserved (typically by a deep-learning framework's caching allocator sized to
 // the whole device), or code on a latency-critical path where cudaMalloc / cudaFree and their implicit
-// device-wide synchronisation are not acceptable.  The regular neox_layernorm_bwd() asks such callers for
-// a scratch buffer they cannot supply; this variant carries its scratch inside the library image instead.
+// device-wide synchronisation are not acceptable.  The regular entry points, neox_layernorm_bwd() and
+// its form with an addend that the framework itself calls, ask such callers for a scratch buffer they cannot supply; this variant carries its scratch inside the library image instead.
 //
 //   int neox_layernorm_bwd_noalloc(g, x, gamma, mean, rstd, dx, dgamma, dbeta, rows, cols, dtype, stream)
 //

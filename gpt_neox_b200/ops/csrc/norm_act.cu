@@ -155,9 +155,9 @@ __device__ __forceinline__ void block_sum2(float& a, float& b, float2 (&red)[32]
 // warp each (no barrier at all, 16 to 32 rows in flight on an SM), longer rows to a CTA with one barrier per reduction.
 // V, the vectors of 8 elements a thread holds, is a template parameter so that a thread keeps registers only for what it
 // has; with room for 4 compiled in throughout, 768-column rows ran at 18 % of the copy bandwidth backward and 20 % forward.
-// In both forms the next row is requested before this row's reductions.  Replayed, before and now, 8192 rows: 768 columns
-// forward 17 -> 8.0 us; 6144 columns forward 55 -> 43 (31 of bytes), backward 106 -> 90 (46) and with addend 187 -> 108 (61);
-// 4096, RMS 35 -> 24, 94 -> 60 and 149 -> 81; 5781 rows of 1024 forward 14.2 -> 7.2.
+// In both forms the next row is requested before this row's reductions.  Replayed, before and now: 16384 rows of 768
+// forward 34 -> 10 us; 8192 rows of 6144 forward 55 -> 43 (31 of bytes), backward 106 -> 90 (46) and with addend 187 -> 108 (61);
+// of 4096, RMS, 35 -> 24, 94 -> 60 and 149 -> 81; 5781 rows of 1024 forward 14.2 -> 7.2.
 constexpr int ROW_WARPS = 8;          // rows of up to 1024 columns: warps (rows) per CTA
 constexpr int ROW_COLS = 1024;
 constexpr int CTA_THREADS = 384;      // longer rows: V = ceil(vectors / 384), 1 to 3; V = 0 re-reads the row instead

@@ -152,8 +152,8 @@ class _collector_rests:
 class GraphDecoder:
     """Token-by-token decoding with a fixed-capacity key/value cache, replayed from a CUDA graph.
 
-    A decoding step of the ordinary cached path launches a few dozen small kernels per layer whose shapes change with
-    the position (the cache grows), so it is bound by launch overhead and cannot be captured.  Here every attention
+    A decoding step of the ordinary cached path makes eight launches per layer whose arguments change with the position (the
+    cache grows), so it is bound by the host work around them and cannot be captured.  Here every attention
     layer owns a ``[2, capacity, batch, heads, d]`` buffer and reads the current position from a device scalar: the
     step's launch sequence is identical for every token, is captured once after the prompt pass and replayed.  On a
     machine without CUDA (or with ``capture=False``) the same static-cache step runs eagerly, which is how its
