@@ -670,11 +670,11 @@ int launch_bwd2(const CUtensorMap* t, const Bwd2Params& p, cudaStream_t st) {
             return NEOX_ERR_LAUNCH;
         attr = true;
     }
-    const long long gkv = (long long)p.kv_order.tiles * p.kv_order.heads, gq = (long long)p.q_order.tiles * p.q_order.heads;
-    if (gkv > 0x7fffffff || gq > 0x7fffffff) return NEOX_ERR_SHAPE;
-    flash_bwd2_dkv_kernel<D, FP16><<<(int)gkv, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
+    dim3 gkv, gq;
+    if (!tile_grid(p.kv_order, gkv.x, gkv.y) || !tile_grid(p.q_order, gq.x, gq.y)) return NEOX_ERR_SHAPE;
+    flash_bwd2_dkv_kernel<D, FP16><<<gkv, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
     if (cudaGetLastError() != cudaSuccess) return NEOX_ERR_LAUNCH;
-    flash_bwd2_dq_kernel<D, FP16><<<(int)gq, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
+    flash_bwd2_dq_kernel<D, FP16><<<gq, THREADS, B2Cfg<D>::SMEM, st>>>(t[0], t[1], t[2], t[3], p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 

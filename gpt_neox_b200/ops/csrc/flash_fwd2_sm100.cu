@@ -529,9 +529,9 @@ int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
             return NEOX_ERR_LAUNCH;
         attr = true;
     }
-    const long long grid = (long long)p.order.tiles * p.order.heads;
-    if (grid > 0x7fffffff) return NEOX_ERR_SHAPE;
-    flash_fwd2_kernel<D, FP16><<<(int)grid, THREADS, Cfg2<D>::SMEM, st>>>(tq, tk, tv, p);
+    dim3 grid;
+    if (!tile_grid(p.order, grid.x, grid.y)) return NEOX_ERR_SHAPE;
+    flash_fwd2_kernel<D, FP16><<<grid, THREADS, Cfg2<D>::SMEM, st>>>(tq, tk, tv, p);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 

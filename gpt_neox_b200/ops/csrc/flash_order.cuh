@@ -12,15 +12,30 @@
 
 struct TileOrder {
     int tiles, heads, group;
+    int plane;              // one group of all heads: the grid is heads x tiles, and a CTA's place needs no division
 };
 
 inline TileOrder tile_order(int tiles, int heads, long long bytes_per_head) {
     const long long fit = (48ll << 20) / (bytes_per_head > 0 ? bytes_per_head : 1);
-    return TileOrder{tiles, heads, (int)(fit < 1 ? 1 : fit < heads ? fit : heads)};
+    const int group = (int)(fit < 1 ? 1 : fit < heads ? fit : heads);
+    return TileOrder{tiles, heads, group, group == heads && tiles <= 65535};
+}
+
+// The grid of an order; false: more CTAs than a grid takes.
+inline bool tile_grid(const TileOrder& o, unsigned& x, unsigned& y) {
+    const long long all = (long long)o.tiles * o.heads;
+    x = (unsigned)(o.plane ? o.heads : all);
+    y = (unsigned)(o.plane ? o.tiles : 1);
+    return all <= 0x7fffffff;
 }
 
 // rank: 0 for the tile to start first.
 __device__ __forceinline__ void pick_tile(const TileOrder& o, int& rank, int& head) {
+    if (o.plane) {
+        rank = blockIdx.y;
+        head = blockIdx.x;
+        return;
+    }
     const int per = o.group * o.tiles, g = blockIdx.x / per, r = blockIdx.x - g * per;
     const int size = min(o.group, o.heads - g * o.group);
     rank = r / size;

@@ -364,7 +364,7 @@ def test_attention_tile_order_starts_every_tile_once(tmp_path):
 using std::min;
 #define __device__
 #define __forceinline__ inline
-static struct { int x; } blockIdx;
+static struct { unsigned x, y; } blockIdx;
 #include "flash_order.cuh"
 int main() {
     const int tiles[] = {1, 3, 16, 64}, heads[] = {1, 2, 8, 17, 256};
@@ -372,7 +372,9 @@ int main() {
     for (int t : tiles) for (int h : heads) for (long long b : bytes) {
         const TileOrder o = tile_order(t, h, b);
         std::printf("%d %d %lld %d", t, h, b, o.group);
-        for (blockIdx.x = 0; blockIdx.x < t * h; ++blockIdx.x) {
+        unsigned gx, gy;
+        if (!tile_grid(o, gx, gy)) return 1;
+        for (blockIdx.y = 0; blockIdx.y < gy; ++blockIdx.y) for (blockIdx.x = 0; blockIdx.x < gx; ++blockIdx.x) {
             int rank, head;
             pick_tile(o, rank, head);
             std::printf(" %d,%d", rank, head);
