@@ -543,10 +543,12 @@ norm_bwd_rows_kernel(const T* __restrict__ g, const T* __restrict__ x, const T* 
     }
 }
 
-// out0[c] (+)= sum_r partial[r][c], out1[c] (+)= sum_r partial[nblk + r][c].  A CTA owns 32 columns; its 32 warps take
-// every 32nd partial row (coalesced 128-byte reads), then the 32 row lanes are added in a fixed order.  The loads of a
-// thread are serial, so what counts is how few each has: 10 of 296 rows; with 8 warps (37 rows) it took 6.1 us.
-constexpr int RED_WARPS = 32;
+// out0[c] (+)= sum_r partial[r][c], out1[c] (+)= sum_r partial[nblk + r][c].  A CTA owns 32 columns; its 32 (8) warps take
+// every 32nd (8th) partial row (coalesced 128-byte reads), then the row lanes are added in a fixed order.  The loads of a
+// thread are serial, so what counts is how few each has: 10 of 296 rows; with 8 warps (37 rows) it took 6.1 us.  Where the
+// columns give every SM two CTAs all the same, 8 warps are enough and more CTAs fit: 100 rows of 16384, both passes of a
+// LayerNorm, 42.8 us with 32 warps and 40.8 with 8.
+template <int RED_WARPS>
 __global__ void __launch_bounds__(RED_WARPS * 32)
 colreduce_kernel(const float* __restrict__ partial, float* __restrict__ out0, float* __restrict__ out1, int nblk, int cols,
                  int acc0, int acc1) {
@@ -658,7 +660,9 @@ int launch_norm_bwd(const void* g, const void* x, const void* gamma, const float
     if (dtype == 0) launch_norm_bwd_t<__nv_bfloat16, RMS>(g, x, gamma, s0, s1, dx, ws, rows, cols, eps, st, add, nblk);
     else if (dtype == 1) launch_norm_bwd_t<float, RMS>(g, x, gamma, s0, s1, dx, ws, rows, cols, eps, st, add, nblk);
     else launch_norm_bwd_t<__half, RMS>(g, x, gamma, s0, s1, dx, ws, rows, cols, eps, st, add, nblk);
-    colreduce_kernel<<<(cols + 31) / 32, RED_WARPS * 32, 0, st>>>(ws, d0, d1, nblk, cols, acc0, acc1);
+    const int cblk = (cols + 31) / 32;
+    if (cblk >= 2 * neox_sm_count()) colreduce_kernel<8><<<cblk, 8 * 32, 0, st>>>(ws, d0, d1, nblk, cols, acc0, acc1);
+    else colreduce_kernel<32><<<cblk, 32 * 32, 0, st>>>(ws, d0, d1, nblk, cols, acc0, acc1);
     return cudaGetLastError() == cudaSuccess ? 0 : NEOX_ERR_LAUNCH;
 }
 
