@@ -45,10 +45,8 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf
 // ckpt and the adjoint's counterpart are [b][chunk][state][channel]: a warp's accesses are whole lines.
 __device__ __forceinline__ size_t slot(int b, int ck, int nchk, int d) { return ((size_t)b * nchk + ck) * NS * d; }
 
-// rows: how many of the chunk's are read later; those past `steps` are zero.
-__device__ __forceinline__ void stage_rows(float (*dst)[NS], const float* __restrict__ src, int steps, long long stride,
-                                           int rows = CHUNK) {
-    for (int i = threadIdx.x; i < rows * NS; i += blockDim.x) {
+__device__ __forceinline__ void stage_rows(float (*dst)[NS], const float* __restrict__ src, int steps, long long stride) {
+    for (int i = threadIdx.x; i < CHUNK * NS; i += blockDim.x) {
         const int s = i / NS, j = i % NS;
         dst[s][j] = s < steps ? src[s * stride + j] : 0.f;
     }
@@ -163,8 +161,8 @@ scan_out_kernel(const bf16* __restrict__ u, const bf16* __restrict__ dt, const f
     for (int ck = first; ck < last; ++ck) {
         const int t0 = ck * CHUNK, steps = min(CHUNK, l - t0);
         __syncthreads();
-        stage_rows(sB, B + b * st.bb + t0 * st.bt, steps, st.bt, steps);
-        stage_rows(sC, C + b * st.cb + t0 * st.ct, steps, st.ct, steps);
+        stage_rows(sB, B + b * st.bb + t0 * st.bt, steps, st.bt);
+        stage_rows(sC, C + b * st.cb + t0 * st.ct, steps, st.ct);
         __syncthreads();
         if (!live) continue;
         if (ck > first) {
